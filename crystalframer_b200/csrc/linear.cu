@@ -6,8 +6,9 @@
 // The problems are small and skinny -- M = atoms of the batch (a few thousand), K and N in {128, 512} -- so a
 // single product is a few microseconds of FP32 work and what matters is (i) that the launches come from one
 // host call per layer instead of one framework dispatch each, (ii) enough thread blocks to cover the SMs,
-// and (iii) epilogues (bias, residual, ReLU and its mask) fused in.  FP32 accumulation on the FMA pipe keeps
-// the 1e-4 tolerance of the path without an error-compensated split.
+// and (iii) epilogues (bias, residual, ReLU and its mask) fused in.  Batches of 512 atoms or more run on the tensor cores
+// (tc_linear.cu); what follows are the kernels of the FP32 pipe, for smaller ones, for shapes that are not whole tiles, and
+// for results that must not depend on how their sums are formed.
 //
 // gemm_kernel<B_KN, TM>:  C[M,N] = sum over up to three products A_s[M,K_s] op(B_s) (+ bias) (+ residual),
 //   then ReLU or a ReLU mask.  B_KN = false: B is [N,K] (a torch Linear weight; forward), true: B is [K,N]
@@ -43,6 +44,26 @@ struct GemmArgs {
 // splits: blocks of a cluster that share a tile's contraction (the product of a block is blockIdx.z / splits); whole: one
 // block each, in one chain of additions whatever the number of tiles
 struct GemmBatch { GemmArgs g[3]; int n, splits, whole; };
+
+// four outputs of row m, from column n on: bias, residual, ReLU, ReLU mask, store
+__device__ __forceinline__ void gemm_finish(const GemmArgs& G, const int m, const int n, float4 v)
+{
+    if (n >= G.N || m >= G.M) return;
+    if (G.bias != nullptr) {
+        const float4 b = __ldg(reinterpret_cast<const float4*>(G.bias + n));
+        v.x += b.x; v.y += b.y; v.z += b.z; v.w += b.w;
+    }
+    if (G.resid != nullptr) {
+        const float4 r = __ldg(reinterpret_cast<const float4*>(G.resid + (size_t)m * G.ldr + n));
+        v.x += r.x; v.y += r.y; v.z += r.z; v.w += r.w;
+    }
+    if (G.relu) { v.x = fmaxf(v.x, 0.f); v.y = fmaxf(v.y, 0.f); v.z = fmaxf(v.z, 0.f); v.w = fmaxf(v.w, 0.f); }
+    if (G.mask != nullptr) {
+        const float4 h = __ldg(reinterpret_cast<const float4*>(G.mask + (size_t)m * G.ldm + n));
+        v.x = h.x > 0.f ? v.x : 0.f; v.y = h.y > 0.f ? v.y : 0.f; v.z = h.z > 0.f ? v.z : 0.f; v.w = h.w > 0.f ? v.w : 0.f;
+    }
+    *reinterpret_cast<float4*>(G.C + (size_t)m * G.ldc + n) = v;
+}
 
 template <bool B_KN, int TM>
 __global__ void __launch_bounds__(kGmThreads) gemm_kernel(const GemmBatch Gb)
@@ -139,23 +160,7 @@ __global__ void __launch_bounds__(kGmThreads) gemm_kernel(const GemmBatch Gb)
     }
 
     const int n = n0 + tx * 4;
-    auto finish = [&](const int m, float4 v) {
-        if (n >= G.N || m >= G.M) return;
-        if (G.bias != nullptr) {
-            const float4 b = __ldg(reinterpret_cast<const float4*>(G.bias + n));
-            v.x += b.x; v.y += b.y; v.z += b.z; v.w += b.w;
-        }
-        if (G.resid != nullptr) {
-            const float4 r = __ldg(reinterpret_cast<const float4*>(G.resid + (size_t)m * G.ldr + n));
-            v.x += r.x; v.y += r.y; v.z += r.z; v.w += r.w;
-        }
-        if (G.relu) { v.x = fmaxf(v.x, 0.f); v.y = fmaxf(v.y, 0.f); v.z = fmaxf(v.z, 0.f); v.w = fmaxf(v.w, 0.f); }
-        if (G.mask != nullptr) {
-            const float4 h = __ldg(reinterpret_cast<const float4*>(G.mask + (size_t)m * G.ldm + n));
-            v.x = h.x > 0.f ? v.x : 0.f; v.y = h.y > 0.f ? v.y : 0.f; v.z = h.z > 0.f ? v.z : 0.f; v.w = h.w > 0.f ? v.w : 0.f;
-        }
-        *reinterpret_cast<float4*>(G.C + (size_t)m * G.ldc + n) = v;
-    };
+    auto finish = [&](const int m, const float4 v) { gemm_finish(G, m, n, v); };
     if (Gb.splits == 1) {
 #pragma unroll
         for (int i = 0; i < TM; i++) finish(m0 + ty * TM + i, make_float4(acc[i][0], acc[i][1], acc[i][2], acc[i][3]));
@@ -213,17 +218,11 @@ static int launch_gemm(GemmBatch& Gb, cudaStream_t st)
 static inline bool gm_aligned(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; }
 
 struct WgArgs;
-static int tc_gemm_batch(const GemmBatch& Gb, bool b_kn, cudaStream_t st);
+struct WgProblem;
+static int tc_gemm_batch(GemmBatch& Gb, bool b_kn, cudaStream_t st);
 static bool tc_gemm_covers(const GemmBatch& Gb);
+static bool tc_wgrad_covers(const WgProblem& Pb, int64_t M);
 static int tc_wgrad_launch(const WgArgs& W, int tiles, cudaStream_t st);
-
-// CFB200_TC=0 keeps the dense layers on the FP32 pipe (gemm_kernel); default: tensor cores where the shapes allow
-static bool use_tensor_cores()
-{
-    static int v = -1;
-    if (v < 0) { const char* e = getenv("CFB200_TC"); v = e ? atoi(e) : 0; }
-    return v != 0;
-}
 
 static int gemm_check(const GemmArgs& G)
 {
@@ -247,7 +246,7 @@ static int gemm_batch(GemmBatch& Gb, bool b_kn, cudaStream_t st)
         const int rc = gemm_check(Gb.g[i]);
         if (rc != CFB200_OK) return rc;
     }
-    if (use_tensor_cores() && tc_gemm_covers(Gb)) return tc_gemm_batch(Gb, b_kn, st);
+    if (tc_gemm_covers(Gb)) return tc_gemm_batch(Gb, b_kn, st);
     // The 64-row tile when with it every SM gets a block, else the 32-row tile (twice the blocks): it reads 8 instead of 6
     // shared-memory cycles for twice the products.  2 273 atoms, [512] -> [128]: 64 rows in four parts against 32 rows in
     // four parts 22.8 us.
@@ -451,7 +450,7 @@ static int64_t wgrad_workspace_floats(int64_t M, int64_t outputs)
 }
 
 // Fills tile counts and scratch offsets, then launches the grouped products and the reduction.  Problems whose
-// output is a whole number of 128 x 128 tiles go to the tensor-core kernel (tc_linear.cu), the others (the per-head
+// output is a whole number of 128 x 64 tiles go to the tensor-core kernel (tc_linear.cu), the others (the per-head
 // value-encoding weights, 16 rows) to wgrad_kernel; both leave their partials in the same scratch layout.
 static int wgrad(WgArgs& W, int64_t ws_floats, cudaStream_t st)
 {
@@ -475,13 +474,12 @@ static int wgrad(WgArgs& W, int64_t ws_floats, cudaStream_t st)
     int tc_tiles = 0, fp_tiles = 0;
     for (int i = 0; i < W.nprob; i++) {
         const WgProblem& Pb = W.prob[i];
-        const bool on_tc = use_tensor_cores() && Pb.nb == 1 && Pb.P % 128 == 0 && Pb.Q % 128 == 0;
+        const bool on_tc = tc_wgrad_covers(Pb, W.M);
         WgArgs& dst = on_tc ? tc : fp;
         WgProblem& q = dst.prob[dst.nprob++];
         q = Pb;
-        const int tile = on_tc ? 128 : kWgTile;
-        q.tiles_p = (Pb.P + tile - 1) / tile;
-        q.tiles_q = (Pb.Q + tile - 1) / tile;
+        q.tiles_p = on_tc ? Pb.P / 128 : (Pb.P + kWgTile - 1) / kWgTile;
+        q.tiles_q = (Pb.Q + kWgTile - 1) / kWgTile;                 // 64 columns either way
         int& tiles = on_tc ? tc_tiles : fp_tiles;
         q.tile0 = tiles;
         tiles += Pb.nb * q.tiles_p * q.tiles_q;

@@ -1,68 +1,107 @@
-// The dense layers on the 5th-generation tensor cores: tcgen05.mma (kind::tf32) with FP32 accumulation in
-// tensor memory, and an error-compensated three-product split so that the results keep FP32 accuracy
-// (the path's tolerance is 1e-4 relative; a single TF32 product has a 10-bit mantissa).
+// The dense layers on the 5th-generation tensor cores: tcgen05.mma (kind::f16, bf16 operands) with FP32 accumulation in
+// tensor memory.  Every operand is split exactly into three bf16 numbers, and six of the nine products are formed:
 //
-//   x = hi + lo,  hi = x with the low 13 mantissa bits cleared (exactly a TF32 number),  lo = x - hi (exact in FP32)
-//   A B^T  ~  A_hi B_hi^T + A_hi B_lo^T + A_lo B_hi^T        (the dropped lo x lo term is below 2^-20 relative)
+//   x = x0 + x1 + x2 (8 significant bits each)
+//   A B^T  ~  A0 B0^T + (A0 B1^T + A1 B0^T + A1 B1^T + A0 B2^T + A2 B0^T)      (what is dropped is below 2^-24 of a product)
 //
-// One CTA of 256 threads owns a 128 x 128 output tile.  Per 32-wide slice of the contraction index the threads
-// bring both operands from global memory through registers (three register sets: two slices' loads are in flight
-// behind the one in work), split them, and store hi and lo parts to one of two shared-memory stages in the
-// K-major, 128-byte-swizzled layout the tensor core reads (8-row groups of 1024 bytes, the 16-byte chunk j of row
-// r stored at chunk j ^ (r & 7)); operands whose contraction index is not contiguous in global memory (the weight
-// in a data gradient, both operands of a weight gradient) are transposed by that staging.  One thread then issues
-// 4 (k-steps of 8) x 3 (products) tcgen05.mma instructions and commits them to the stage's mbarrier, which is
-// waited on before the stage is written again two slices later.  The epilogue reads the accumulator with
-// tcgen05.ld (a warp reads the TMEM lanes of its quarter: rows; warps w and w + 4 take half of the columns each),
-// applies bias / residual / ReLU / ReLU mask and stores.  Every wait on the mbarrier is bounded: on expiry the kernel sets CFB200_ST_TC_TIMEOUT, frees its
-// tensor memory and returns.
+// at the price of three TF32 products, whose two parts lose two bits of an operand.
+// Accuracy: the tensor core cuts off what does not fit when it adds to its accumulator, so one accumulator for everything
+// would collect an error of one sign per instruction.  The A0 B0 products therefore go in turns to three accumulators and
+// the small products to a fourth; the epilogue adds the four in FP32.  Distance from 64 bits, of the result's norm, for
+// normal operands and 128 / 512 terms: 6.6e-8 / 7.8e-8 (16e-8 where one block takes all 512); a chain of FP32 fused
+// multiply-adds 20e-8 / 21e-8 (41e-8), three TF32 products 16e-8 / 16e-8 (44e-8).  Operands of one sign, and ReLU outputs,
+// fare no worse (6.8e-8 against 16e-8, 5.4e-8 against 14e-8).
 //
-// No TMA: the operands need the hi / lo split on the way to shared memory, so they pass through registers anyway.
+// One CTA of eight warps and one owns a 128 x 64 output tile (or, over a cluster, a part of its contraction).  Per 32-wide slice
+// of the contraction index the eight warps bring both operands from global memory through registers (two register sets:
+// a slice's loads are in flight behind the one in work), split them, and store the three parts to one of three
+// shared-memory stages as they lie in global memory, in the layout the tensor core reads: operands whose contraction index
+// is contiguous K-major with 64-byte swizzle (8-row groups of 512 bytes, the 16-byte chunk j of row r stored at chunk
+// j ^ ((r >> 1) & 3)), the others (the weight in a data gradient, both operands of a weight gradient) MN-major with 128-byte
+// swizzle (blocks of 64 rows; a contraction index is 128 bytes, its chunk j stored at chunk j ^ (k & 7)).  A thread of the
+// ninth warp waits for the stage to be full (an mbarrier that each warp arrives at), issues 2 (k-steps of 16) x 6 (products)
+// tcgen05.mma instructions and commits them to the stage's other mbarrier, which is waited on before the stage is written
+// again three slices later: nobody else waits for the tensor core, whose queue holds up the thread that fills it.  The
+// epilogue adds the accumulators (tcgen05.ld; a warp reads the TMEM lanes of its quarter: rows; warps w and w + 4 take half
+// of the columns each), leaves the tile in shared memory, and finishes it row by row: bias, residual, ReLU, ReLU mask.
+//
+// Two CTAs fit an SM (109 KB of shared memory, half of the tensor memory, 96 registers a thread): one splits while the
+// other multiplies.  Every kernel here that allocates tensor memory needs as much, so an allocation never waits.
+// What bounds it: up to 2 700 rows a chain of latencies (launch, first loads, four slices, epilogue), beyond that the
+// instructions of the split (issue slots 48 % busy, tensor pipe 18 %).  Kernel time, [128] -> [512] and [512] -> [128],
+// against FP32 in gemm_kernel: 400 rows 7.5 / 8.9 against 7.1 / 8.6 us, 600 rows 7.6 / 9.0 against 10.3 / 11.9, 2 661 rows
+// 10.6 / 12.0 against 17.4 / 19.3, 10 700 rows 25 / 25 against 52 / 59; weight gradients of a layer of 10 700 atoms 64 against
+// 190.  Measured and left: 16 warps that bring and split, and a block barrier per slice with the instructions issued by one
+// of them (27 / 29 us); operands transposed on their way to shared memory (27 / 35 us in data gradients).
+//
+// Every wait on an mbarrier is bounded: on expiry the kernel sets CFB200_ST_TC_TIMEOUT, goes on with wrong numbers and
+// ends.  An operand that is not finite has no split (inf - inf); a tile with a result that is not finite is computed again
+// in plain FP32.
+//
+// No TMA: the operands need the split on the way to shared memory, so they pass through registers anyway.
 #include <atomic>
+#include <cuda_bf16.h>
 #include "common.cuh"
 
 namespace cfb {
 
-constexpr int kTcThreads = 256;
-constexpr int kTcTile = 128;                 // rows of either operand per tile
-constexpr int kTcKc = 32;                    // contraction slice: 32 floats = one 128-byte swizzle row
-constexpr int kTcOperandBytes = kTcTile * kTcKc * 4;            // 16 KB
-constexpr int kTcStageBytes = 4 * kTcOperandBytes;              // A hi, A lo, B hi, B lo
-constexpr int kTcSmemBytes = 2 * kTcStageBytes + 1024;          // two stages + alignment slack
+constexpr int kTcThreads = 256;              // that bring and split operands, and finish the tile
+constexpr int kTcBlock = kTcThreads + 32;    // and the warp that issues the tensor core's instructions
+constexpr int kTcM = 128, kTcN = 64;         // rows of the operands per tile
+constexpr int kTcKc = 32;                    // contraction slice: 32 bf16 = one 64-byte swizzle row
+constexpr int kTcABytes = kTcM * kTcKc * 2, kTcBBytes = kTcN * kTcKc * 2;       // one part: 8 KB, 4 KB
+constexpr int kTcStageBytes = 3 * (kTcABytes + kTcBBytes);      // A0, A1, A2, B0, B1, B2
+constexpr int kTcStages = 3;
+constexpr int kTcSmemBytes = kTcStages * kTcStageBytes + 1024;  // and alignment slack
+constexpr int kTcAcc = 3;                    // accumulators of the large products; the small ones' follows them
+constexpr int kTcCols = 256;                 // tensor-memory columns: four accumulators
+constexpr int kTcTileLd = kTcN / 4 + 1;      // float4 per row of the finished tile (conflict-free writes by rows)
+static_assert((kTcM * kTcTileLd + kTcThreads) * 16 <= kTcStages * kTcStageBytes, "the finished tile, and column sums, fit the stages");
 constexpr uint32_t kTcSpinLimit = 1u << 22;
 
 __device__ __forceinline__ uint32_t smem_u32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
 
-// byte offset of the 16-byte chunk j (0..7) of row r (0..127) in a K-major 128-byte-swizzled operand tile
-__device__ __forceinline__ uint32_t tc_chunk_offset(int r, int j)
+// Two numbers into three bf16 each (packed: x low, y high); every step is exact.  A number that is not finite, or rounds to
+// infinity, leaves a part that is not a number.
+__device__ __forceinline__ void tc_split2(float x, float y, uint32_t (&part)[3])
 {
-    return (uint32_t)((r >> 3) * 1024 + (r & 7) * 128 + ((j ^ (r & 7)) << 4));
+#pragma unroll
+    for (int i = 0; i < 3; i++) {
+        const __nv_bfloat162 b = __floats2bfloat162_rn(x, y);
+        part[i] = *reinterpret_cast<const uint32_t*>(&b);
+        if (i < 2) { x -= __uint_as_float(part[i] << 16); y -= __uint_as_float(part[i] & 0xFFFF0000u); }
+    }
 }
 
-__device__ __forceinline__ void tc_split(const float x, float& hi, float& lo)
-{
-    hi = __uint_as_float(__float_as_uint(x) & 0xFFFFE000u);
-    lo = x - hi;
-}
-
-// shared-memory matrix descriptor: K-major, SWIZZLE_128B, 8-row groups 1024 bytes apart, descriptor version 1
+// Shared-memory matrix descriptor, version 1.  K-major, SWIZZLE_64B: 8-row groups 512 bytes apart.  MN-major (TR),
+// SWIZZLE_128B: blocks of 64 rows kTcKc x 128 bytes apart, 8 contraction indices 1024 bytes apart.
+template <bool TR>
 __device__ __forceinline__ uint64_t tc_smem_desc(uint32_t saddr)
 {
-    return (uint64_t)((saddr & 0x3FFFF) >> 4) | ((uint64_t)1 << 16) | ((uint64_t)(1024 >> 4) << 32) | ((uint64_t)1 << 46) |
-           ((uint64_t)2 << 61);
+    const uint64_t base = (uint64_t)((saddr & 0x3FFFF) >> 4) | ((uint64_t)1 << 46);
+    if (TR) return base | ((uint64_t)(kTcKc * 128 >> 4) << 16) | ((uint64_t)(1024 >> 4) << 32) | ((uint64_t)2 << 61);
+    return base | ((uint64_t)1 << 16) | ((uint64_t)(512 >> 4) << 32) | ((uint64_t)4 << 61);
 }
 
-// instruction descriptor: D = F32, A = B = TF32, both K-major, M = 128, N = 128
-constexpr uint32_t kTcIdesc = (1u << 4) | (2u << 7) | (2u << 10) | ((uint32_t)(kTcTile >> 3) << 17) | ((uint32_t)(kTcTile >> 4) << 24);
+// from one k-step of 16 to the next, in descriptor units of 16 bytes
+__host__ __device__ constexpr uint64_t tc_kstep(bool TR) { return TR ? 2 * 1024 >> 4 : 32 >> 4; }
 
-__device__ __forceinline__ void tc_mma(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc, uint32_t accumulate)
+// instruction descriptor: D = F32, A = B = BF16, M = 128, N = 64; bits 15, 16: A, B MN-major
+template <bool TRA, bool TRB>
+__device__ __forceinline__ constexpr uint32_t tc_idesc()
+{
+    return (1u << 4) | (1u << 7) | (1u << 10) | ((TRA ? 1u : 0u) << 15) | ((TRB ? 1u : 0u) << 16) | ((uint32_t)(kTcN >> 3) << 17) |
+           ((uint32_t)(kTcM >> 4) << 24);
+}
+
+__device__ __forceinline__ void tc_mma(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc, uint32_t idesc, uint32_t accumulate)
 {
     asm volatile(
         "{\n\t"
         ".reg .pred p;\n\t"
         "setp.ne.b32 p, %4, 0;\n\t"
-        "tcgen05.mma.cta_group::1.kind::tf32 [%0], %1, %2, %3, {%5, %5, %5, %5}, p;\n\t"
-        "}\n" ::"r"(tmem_d), "l"(adesc), "l"(bdesc), "r"(kTcIdesc), "r"(accumulate), "r"(0u)
+        "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, {%5, %5, %5, %5}, p;\n\t"
+        "}\n" ::"r"(tmem_d), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate), "r"(0u)
         : "memory");
 }
 
@@ -80,60 +119,71 @@ __device__ __forceinline__ bool tc_wait(uint32_t mbar, uint32_t parity)
     return false;
 }
 
-// One operand of a product: element (r, k) of the (rows x K) operand is src[r * ld + k] (k contiguous), or, when
-// `transposed`, src[k * ld + r].
-struct TcOperand { const float* src; int ld; int rows; int transposed; };
+// registers holding one slice of both operands
+__host__ __device__ constexpr int tc_float4(int rows) { return rows * kTcKc / 4 / kTcThreads; }
+struct TcSlice { float4 a[tc_float4(kTcM)], b[tc_float4(kTcN)]; };
 
-// registers holding one 128 x 32 slice of both operands: 4 float4 per thread and operand
-struct TcSlice { float4 a[4], b[4]; };
-
-__device__ __forceinline__ void tc_fetch1(float4* v, const TcOperand& Op, const int r0, const int k0, const int K, const int tid)
-{
-    const int warp = tid >> 5, lane = tid & 31;
+// One operand of a product as one thread fetches it.  Element (r, k) of the operand is src[r * ld + k] (k contiguous) or,
+// transposed, src[k * ld + r].  The thread's float4 i of a slice is number tid + 256 i, eight to a row of K or,
+// transposed, ROWS / 4 to a contraction index: from one to the next are 32 rows, or 1024 / ROWS indices.
+template <int ROWS, bool TR>
+struct TcFetch {
+    static constexpr int kSkip = TR ? kTcThreads * 4 / ROWS : kTcThreads / 8;    // rows or indices from one float4 to the next
+    const float* p;                          // the thread's first float4 of the slice to fetch next
+    int step, stride;                        // to the next slice, to the next float4
+    int left;                                // rows (transposed: contraction indices) from the thread's first on
+    __device__ __forceinline__ static int row() { return TR ? 4 * ((int)threadIdx.x % (ROWS / 4)) : (int)threadIdx.x >> 3; }
+    __device__ __forceinline__ static int idx() { return TR ? (int)threadIdx.x / (ROWS / 4) : 4 * ((int)threadIdx.x & 7); }
+    // operand rows r0 .. and contraction indices k0 .. on; rows: of the operand.  Transposed: all of its rows exist, and
+    // contraction indices up to K do; else all indices of a slice exist
+    __device__ __forceinline__ void open(const float* src, const int ld, const int r0, const int rows, const int k0, const int K)
+    {
+        const size_t r = r0 + row(), k = k0 + idx();
+        p = src + (TR ? k * ld + r : r * ld + k);
+        step = TR ? kTcKc * ld : kTcKc;
+        stride = kSkip * ld;
+        left = TR ? K - (int)k : rows - (int)r;
+    }
+    __device__ __forceinline__ void next(float4* v)
+    {
 #pragma unroll
-    for (int i = 0; i < 4; i++) {
-        float4 x = make_float4(0.f, 0.f, 0.f, 0.f);
-        if (!Op.transposed) {
-            const int q = tid + kTcThreads * i, r = q >> 3, j = q & 7;           // row r, 16-byte chunk j
-            if (r0 + r < Op.rows && k0 + 4 * j < K) x = __ldg(reinterpret_cast<const float4*>(Op.src + (size_t)(r0 + r) * Op.ld + k0 + 4 * j));
-        } else {
-            const int r = 4 * (warp + 8 * i), k = lane;                          // rows r..r+3 of contraction index k
-            if (r0 + r < Op.rows && k0 + k < K) x = __ldg(reinterpret_cast<const float4*>(Op.src + (size_t)(k0 + k) * Op.ld + r0 + r));
+        for (int i = 0; i < tc_float4(ROWS); i++) {
+            v[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+            if (i * kSkip < left) v[i] = __ldg(reinterpret_cast<const float4*>(p + (ptrdiff_t)i * stride));
         }
-        v[i] = x;
+        p += step;
+        if (TR) left -= kTcKc;
+    }
+    // where the thread's first float4 goes in a part of a stage (half of a 16-byte chunk), and how far the next ones are
+    __device__ __forceinline__ static int place()
+    {
+        const int r = row(), k = idx();
+        return TR ? (r >> 6) * (kTcKc * 128) + k * 128 + ((((r >> 3) ^ k) & 7) << 4) + 2 * (r & 4)
+                  : r * 64 + (((k >> 3) ^ (r >> 1)) & 3) * 16 + 2 * (k & 4);
+    }
+    static constexpr int kNext = kSkip * (TR ? 128 : 64);
+    static_assert(kSkip % 8 == 0, "the swizzle of a thread's float4 is the same");
+};
+
+// splits a slice into its stage, from the thread's place on (the parts of an operand are ROWS * 64 bytes apart)
+template <int ROWS, bool TR>
+__device__ __forceinline__ void tc_stash1(const float4* v, uint8_t* o)
+{
+#pragma unroll
+    for (int i = 0; i < tc_float4(ROWS); i++) {
+        uint32_t lo[3], hi[3];
+        tc_split2(v[i].x, v[i].y, lo);
+        tc_split2(v[i].z, v[i].w, hi);
+#pragma unroll
+        for (int p = 0; p < 3; p++)
+            *reinterpret_cast<uint2*>(o + i * TcFetch<ROWS, TR>::kNext + p * ROWS * 64) = make_uint2(lo[p], hi[p]);
     }
 }
 
-__device__ __forceinline__ void tc_stash1(const float4* v, const TcOperand& Op, uint8_t* hi_base, uint8_t* lo_base, const int tid)
-{
-    const int warp = tid >> 5, lane = tid & 31;
-#pragma unroll
-    for (int i = 0; i < 4; i++) {
-        const float x[4] = {v[i].x, v[i].y, v[i].z, v[i].w};
-        float h[4], l[4];
-#pragma unroll
-        for (int c = 0; c < 4; c++) tc_split(x[c], h[c], l[c]);
-        if (!Op.transposed) {
-            const int q = tid + kTcThreads * i, r = q >> 3, j = q & 7;
-            const uint32_t off = tc_chunk_offset(r, j);
-            *reinterpret_cast<float4*>(hi_base + off) = make_float4(h[0], h[1], h[2], h[3]);
-            *reinterpret_cast<float4*>(lo_base + off) = make_float4(l[0], l[1], l[2], l[3]);
-        } else {
-            const int r = 4 * (warp + 8 * i), k = lane;
-#pragma unroll
-            for (int c = 0; c < 4; c++) {
-                const uint32_t off = tc_chunk_offset(r + c, k >> 2) + (uint32_t)((k & 3) << 2);
-                *reinterpret_cast<float*>(hi_base + off) = h[c];
-                *reinterpret_cast<float*>(lo_base + off) = l[c];
-            }
-        }
-    }
-}
-
-// CTA-wide state of one tile computation: two shared-memory stages, each with the mbarrier its instructions commit to
+// CTA-wide state of one tile computation: the shared-memory stages with their mbarriers
 struct TcCta {
-    uint8_t* stage[2];
-    uint32_t mbar[2], tmem;
+    uint8_t* stage;
+    uint32_t full, empty, tmem;              // mbarriers per stage: written by all warps; read by its instructions
     uint32_t slices_done;
     bool failed;
 };
@@ -141,18 +191,20 @@ struct TcCta {
 __device__ __forceinline__ void tc_begin(TcCta& T, uint8_t* smem_raw, uint64_t* mbar_slots, uint32_t* tmem_slot)
 {
     const uint32_t base = (smem_u32(smem_raw) + 1023u) & ~1023u;
-    uint8_t* aligned = smem_raw + (base - smem_u32(smem_raw));
-    T.stage[0] = aligned; T.stage[1] = aligned + kTcStageBytes;
-    T.mbar[0] = smem_u32(mbar_slots); T.mbar[1] = smem_u32(mbar_slots + 1);
+    T.stage = smem_raw + (base - smem_u32(smem_raw));
+    T.full = smem_u32(mbar_slots);
+    T.empty = T.full + 8 * kTcStages;
     T.slices_done = 0;
     T.failed = false;
     if (threadIdx.x == 0) {
-        asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(T.mbar[0]) : "memory");
-        asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(T.mbar[1]) : "memory");
+        for (int i = 0; i < kTcStages; i++) {
+            asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(T.full + 8 * i), "r"(kTcThreads / 32) : "memory");
+            asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(T.empty + 8 * i) : "memory");
+        }
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     if ((threadIdx.x >> 5) == 0) {
-        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)), "r"((uint32_t)kTcTile) : "memory");
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)), "r"((uint32_t)kTcCols) : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
     }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
@@ -161,235 +213,330 @@ __device__ __forceinline__ void tc_begin(TcCta& T, uint8_t* smem_raw, uint64_t* 
     T.tmem = *tmem_slot;
 }
 
-// Adds one 32-wide slice held in registers to the accumulator: splits it into the stage slices_done & 1 of shared
-// memory (once the instructions that read that stage two slices ago have finished) and issues its instructions.
-__device__ __forceinline__ void tc_slice(TcCta& T, const TcSlice& S, const TcOperand& OpA, const TcOperand& OpB)
+// Splits one 32-wide slice held in registers into the stage slices_done % 3 of shared memory, once the instructions that
+// read that stage three slices ago have finished.
+template <bool TRA, bool TRB>
+__device__ __forceinline__ void tc_slice(TcCta& T, const TcSlice& S)
 {
-    const int tid = threadIdx.x;
-    const uint32_t s = T.slices_done, st = s & 1;
-    if (s >= 2 && !T.failed) {
-        const bool ok = tc_wait(T.mbar[0] + 8 * st, ((s >> 1) - 1) & 1);
-        T.failed = __syncthreads_or(ok ? 0 : 1) != 0;
-    }
-    if (T.failed) return;
-    uint8_t* base = T.stage[0] + st * kTcStageBytes;
-    tc_stash1(S.a, OpA, base, base + kTcOperandBytes, tid);
-    tc_stash1(S.b, OpB, base + 2 * kTcOperandBytes, base + 3 * kTcOperandBytes, tid);
+    const uint32_t s = T.slices_done++, round = s / kTcStages, st = s - round * kTcStages;
+    if (round > 0 && !tc_wait(T.empty + 8 * st, (round - 1) & 1)) T.failed = true;
+    uint8_t* base = T.stage + st * kTcStageBytes;
+    tc_stash1<kTcM, TRA>(S.a, base + TcFetch<kTcM, TRA>::place());
+    tc_stash1<kTcN, TRB>(S.b, base + 3 * kTcABytes + TcFetch<kTcN, TRB>::place());
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");      // generic-proxy stores -> visible to the tensor core
-    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-    __syncthreads();
-    if (tid == 0) {
+    __syncwarp();
+    if ((threadIdx.x & 31) == 0) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(T.full + 8 * st) : "memory");
+}
+
+// One thread of the last warp: the instructions of `total` slices, each when its stage is full.
+template <bool TRA, bool TRB>
+__device__ __forceinline__ void tc_issue(TcCta& T, const int total)
+{
+    constexpr uint32_t idesc = tc_idesc<TRA, TRB>();
+    constexpr uint64_t pa = kTcABytes >> 4, pb = kTcBBytes >> 4;      // from part to part, in descriptor units of 16 bytes
+    const uint32_t small = T.tmem + kTcAcc * kTcN;
+    for (uint32_t s = 0; s < (uint32_t)total; s++) {
+        const uint32_t round = s / kTcStages, st = s - round * kTcStages;
+        if (!tc_wait(T.full + 8 * st, round & 1)) T.failed = true;
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-        const uint64_t ah = tc_smem_desc(smem_u32(base)), al = tc_smem_desc(smem_u32(base + kTcOperandBytes));
-        const uint64_t bh = tc_smem_desc(smem_u32(base + 2 * kTcOperandBytes)), bl = tc_smem_desc(smem_u32(base + 3 * kTcOperandBytes));
+        const uint32_t base = smem_u32(T.stage) + st * kTcStageBytes;
+        const uint64_t a0 = tc_smem_desc<TRA>(base), b0 = tc_smem_desc<TRB>(base + 3 * kTcABytes);
 #pragma unroll
-        for (int k = 0; k < kTcKc / 8; k++) {                         // 8 TF32 values = 32 bytes per instruction: 2 descriptor units
-            const uint64_t adv = (uint64_t)(2 * k);
-            tc_mma(T.tmem, ah + adv, bh + adv, (s > 0 || k > 0) ? 1u : 0u);
-            tc_mma(T.tmem, ah + adv, bl + adv, 1u);
-            tc_mma(T.tmem, al + adv, bh + adv, 1u);
+        for (uint32_t k = 0; k < kTcKc / 16; k++) {
+            const uint64_t a = a0 + k * tc_kstep(TRA), b = b0 + k * tc_kstep(TRB);
+            const uint32_t n = s * (kTcKc / 16) + k;
+            tc_mma(T.tmem + (n % kTcAcc) * kTcN, a, b, idesc, n >= (uint32_t)kTcAcc ? 1u : 0u);
+            tc_mma(small, a, b + pb, idesc, n > 0 ? 1u : 0u);
+            tc_mma(small, a + pa, b, idesc, 1u);
+            tc_mma(small, a + pa, b + pb, idesc, 1u);
+            tc_mma(small, a, b + 2 * pb, idesc, 1u);
+            tc_mma(small, a + 2 * pa, b, idesc, 1u);
         }
-        asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(T.mbar[0] + 8 * st) : "memory");
+        asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(T.empty + 8 * st) : "memory");
     }
-    T.slices_done++;
 }
 
-// Waits for the last slice (its commit covers every instruction issued before it); true if the accumulator is complete.
-__device__ __forceinline__ bool tc_finish(TcCta& T)
-{
-    if (T.slices_done > 0 && !T.failed) {
-        const uint32_t s = T.slices_done - 1;
-        const bool ok = tc_wait(T.mbar[0] + 8 * (s & 1), (s >> 1) & 1);
-        T.failed = __syncthreads_or(ok ? 0 : 1) != 0;
-    }
-    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-    if (T.failed && threadIdx.x == 0) atomicOr(&g_status, CFB200_ST_TC_TIMEOUT);
-    return !T.failed && T.slices_done > 0;
-}
-
-__device__ __forceinline__ void tc_end(TcCta& T)
-{
-    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-    __syncthreads();
-    if ((threadIdx.x >> 5) == 0)
-        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(T.tmem), "r"((uint32_t)kTcTile) : "memory");
-}
-
-// Output row and column range of this thread in the epilogue: a warp may read the TMEM lanes 32 (w & 3) .. + 31
-// only, so warps w and w + 4 share 32 rows and take 64 columns each.
-__device__ __forceinline__ int tc_row() { return ((threadIdx.x >> 5) & 3) * 32 + (threadIdx.x & 31); }
-__device__ __forceinline__ int tc_col0() { return (threadIdx.x >> 7) * (kTcTile / 2); }
-
-// 16 consecutive accumulator columns of this thread's row
-__device__ __forceinline__ void tc_load16(uint32_t tmem, int col, float* v)
+// 16 accumulator columns of this thread's row, from column `col` of tensor memory
+__device__ __forceinline__ void tc_load16(uint32_t (&r)[16], uint32_t tmem, int col)
 {
     const uint32_t addr = tmem + ((uint32_t)(((threadIdx.x >> 5) & 3) * 32) << 16) + (uint32_t)col;
-    uint32_t r[16];
     asm volatile(
-        "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];\n\t"
-        "tcgen05.wait::ld.sync.aligned;\n"
+        "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];\n"
         : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]), "=r"(r[9]),
           "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
         : "r"(addr) : "memory");
+}
+
+// Waits for the last slice (its commit covers every instruction issued before it), adds the accumulators and leaves the tile
+// in shared memory: row r at tile + r * kTcTileLd.  Returns it after a block barrier, tensor memory freed.  exact(m, n):
+// the element in plain FP32, for tiles with results that are not finite.
+template <class Exact>
+__device__ __forceinline__ float4* tc_finish(TcCta& T, const int total, Exact&& exact)
+{
+    float4* tile = reinterpret_cast<float4*>(T.stage);
+    const int row = ((threadIdx.x >> 5) & 3) * 32 + (threadIdx.x & 31), half = threadIdx.x >> 7;
+    if (total > 0) {
+        const uint32_t s = total - 1;
+        if (!tc_wait(T.empty + 8 * (s % kTcStages), (s / kTcStages) & 1)) T.failed = true;
+    }
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    const bool brings = threadIdx.x < kTcThreads;
+    __syncthreads();                                            // every warp knows that the stages are free
+    float seen = 0.f;                                           // of this thread's outputs: finite when they are (or wrongly not)
+    if (brings && total > 0) {
+#pragma unroll 1
+        for (int c = 0; c < 2; c++) {
+            const int c0 = half * 32 + c * 16;
+            uint32_t u[kTcAcc + 1][16];
 #pragma unroll
-    for (int i = 0; i < 16; i++) v[i] = __uint_as_float(r[i]);
+            for (int a = 0; a <= kTcAcc; a++) tc_load16(u[a], T.tmem, a * kTcN + c0);
+            // the loaded values must not be used, or moved, before this wait
+            asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+            for (int a = 0; a <= kTcAcc; a++)
+#pragma unroll
+                for (int i = 0; i < 16; i++) asm volatile("" : "+r"(u[a][i]));
+#pragma unroll
+            for (int q = 0; q < 4; q++) {
+                float v[4];
+#pragma unroll
+                for (int i = 0; i < 4; i++) {
+                    const int x = 4 * q + i;
+                    // (a contraction of one slice of 32 has used two of the three accumulators)
+                    const float third = total > 1 ? __uint_as_float(u[2][x]) : 0.f;
+                    v[i] = ((__uint_as_float(u[0][x]) + __uint_as_float(u[1][x])) + third) + __uint_as_float(u[3][x]);
+                    seen += v[i];
+                }
+                tile[row * kTcTileLd + (c0 >> 2) + q] = make_float4(v[0], v[1], v[2], v[3]);
+            }
+        }
+    }
+    const bool bad = __syncthreads_or(!(fabsf(seen) <= 3.4e38f));
+    if (brings && (total == 0 || bad)) {
+        for (int q = 0; q < 8; q++) {
+            float v[4] = {0.f, 0.f, 0.f, 0.f};
+            if (bad)
+                for (int i = 0; i < 4; i++) v[i] = exact(row, half * 32 + 4 * q + i);
+            tile[row * kTcTileLd + half * 8 + q] = make_float4(v[0], v[1], v[2], v[3]);
+        }
+    }
+    if (T.failed) atomicOr(&g_status, CFB200_ST_TC_TIMEOUT);
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    __syncthreads();
+    if ((threadIdx.x >> 5) == 0)
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(T.tmem), "r"((uint32_t)kTcCols) : "memory");
+    return tile;
 }
 
 // ---- C = sum_s A_s op(B_s) (+ bias) (+ residual), ReLU / mask: same contract as gemm_kernel (linear.cu) ----------
 template <bool B_KN>
-__global__ void __launch_bounds__(kTcThreads, 1) tc_gemm_kernel(const GemmBatch Gb)
+__global__ void __launch_bounds__(kTcBlock, 2) tc_gemm_kernel(const GemmBatch Gb)
 {
     extern __shared__ uint8_t tc_smem[];
-    __shared__ uint64_t mbar_slots[2];
+    __shared__ uint64_t mbar_slots[2 * kTcStages];
     __shared__ uint32_t tmem_slot;
-    const GemmArgs& G = Gb.g[blockIdx.z];
-    const int tid = threadIdx.x;
-    const int m0 = blockIdx.x * kTcTile, n0 = blockIdx.y * kTcTile;
-    TcCta T;
-    tc_begin(T, tc_smem, mbar_slots, &tmem_slot);
+    const GemmArgs& G = Gb.g[blockIdx.z / Gb.splits];
+    const int rank = blockIdx.z % Gb.splits;
+    const int m0 = blockIdx.x * kTcM, n0 = blockIdx.y * kTcN;
     int total = 0;
     for (int s = 0; s < G.nseg; s++) total += G.seg[s].K / kTcKc;
-    TcOperand OA, OB;
-    OA.rows = G.M; OA.transposed = 0; OB.rows = G.N; OB.transposed = B_KN ? 1 : 0;
-    // slice index -> (segment, offset): three register sets keep two slices' loads in flight behind the one in work
-    auto fetch = [&](TcSlice& R, int slice) {
-        if (slice >= total) return;
-        int s = 0;
-        while (slice >= G.seg[s].K / kTcKc) { slice -= G.seg[s].K / kTcKc; s++; }
-        OA.src = G.seg[s].A; OA.ld = G.seg[s].lda; OB.src = G.seg[s].B; OB.ld = G.seg[s].ldb;
-        tc_fetch1(R.a, OA, m0, slice * kTcKc, G.seg[s].K, tid);
-        tc_fetch1(R.b, OB, n0, slice * kTcKc, G.seg[s].K, tid);
+    const int first = total * rank / Gb.splits;                 // this block's share of the slices
+    total = total * (rank + 1) / Gb.splits - first;
+    // the slices one after the other, over the segments; two register sets keep a slice's loads in flight behind the one in
+    // work
+    TcFetch<kTcM, false> FA;
+    TcFetch<kTcN, B_KN> FB;
+    int seg = 0, in_seg = first, ahead = 0;                     // the slice to fetch next: segment, number in it, number
+    while (in_seg >= G.seg[seg].K / kTcKc) in_seg -= G.seg[seg++].K / kTcKc;
+    auto open = [&]() {
+        const GemmSeg& S = G.seg[seg];
+        FA.open(S.A, S.lda, m0, G.M, in_seg * kTcKc, S.K);
+        FB.open(S.B, S.ldb, n0, G.N, in_seg * kTcKc, S.K);
     };
-    TcSlice R0, R1, R2;
-    fetch(R0, 0); fetch(R1, 1); fetch(R2, 2);
-    for (int s = 0; s < total; s += 3) {
-        tc_slice(T, R0, OA, OB); fetch(R0, s + 3);
-        if (s + 1 < total) { tc_slice(T, R1, OA, OB); fetch(R1, s + 4); }
-        if (s + 2 < total) { tc_slice(T, R2, OA, OB); fetch(R2, s + 5); }
-    }
-    if (tc_finish(T)) {
-        const int m = m0 + tc_row();
-        for (int c0 = tc_col0(); c0 < tc_col0() + kTcTile / 2; c0 += 16) {
-            float v[16];
-            tc_load16(T.tmem, c0, v);
-            const int n = n0 + c0;
-            if (m < G.M && n < G.N) {
-#pragma unroll
-                for (int q4 = 0; q4 < 4; q4++) {
-                    float4 o = make_float4(v[4 * q4], v[4 * q4 + 1], v[4 * q4 + 2], v[4 * q4 + 3]);
-                    const int nn = n + 4 * q4;
-                    if (G.bias != nullptr) { const float4 b = __ldg(reinterpret_cast<const float4*>(G.bias + nn)); o.x += b.x; o.y += b.y; o.z += b.z; o.w += b.w; }
-                    if (G.resid != nullptr) {
-                        const float4 r = __ldg(reinterpret_cast<const float4*>(G.resid + (size_t)m * G.ldr + nn));
-                        o.x += r.x; o.y += r.y; o.z += r.z; o.w += r.w;
-                    }
-                    if (G.relu) { o.x = fmaxf(o.x, 0.f); o.y = fmaxf(o.y, 0.f); o.z = fmaxf(o.z, 0.f); o.w = fmaxf(o.w, 0.f); }
-                    if (G.mask != nullptr) {
-                        const float4 hm = __ldg(reinterpret_cast<const float4*>(G.mask + (size_t)m * G.ldm + nn));
-                        o.x = hm.x > 0.f ? o.x : 0.f; o.y = hm.y > 0.f ? o.y : 0.f; o.z = hm.z > 0.f ? o.z : 0.f; o.w = hm.w > 0.f ? o.w : 0.f;
-                    }
-                    *reinterpret_cast<float4*>(G.C + (size_t)m * G.ldc + nn) = o;
-                }
-            }
+    open();
+    auto fetch = [&](TcSlice& R) {
+        if (ahead++ >= total) return;
+        if (in_seg == G.seg[seg].K / kTcKc) { seg++; in_seg = 0; open(); }
+        FA.next(R.a);
+        FB.next(R.b);
+        in_seg++;
+    };
+    TcSlice R0, R1;
+    const bool brings = threadIdx.x < kTcThreads;
+    if (brings) { fetch(R0); fetch(R1); }
+    TcCta T;
+    tc_begin(T, tc_smem, mbar_slots, &tmem_slot);
+    if (brings) {
+        for (int s = 0; s < total; s += 2) {
+            tc_slice<false, B_KN>(T, R0); fetch(R0);
+            if (s + 1 < total) { tc_slice<false, B_KN>(T, R1); fetch(R1); }
         }
+    } else if (threadIdx.x == kTcThreads) {
+        tc_issue<false, B_KN>(T, total);
     }
-    tc_end(T);
+    __syncwarp();
+    float4* tile = tc_finish(T, total, [&](const int r, const int c) {
+        float v = 0.f;
+        const int m = m0 + r, n = n0 + c;
+        if (m >= G.M || n >= G.N) return v;
+        for (int x = first; x < first + total; x++) {
+            int s = 0, k0 = x;
+            while (k0 >= G.seg[s].K / kTcKc) { k0 -= G.seg[s].K / kTcKc; s++; }
+            const GemmSeg& S = G.seg[s];
+            for (int k = k0 * kTcKc; k < (k0 + 1) * kTcKc; k++)
+                v = fmaf(__ldg(S.A + (size_t)m * S.lda + k), __ldg(B_KN ? S.B + (size_t)k * S.ldb + n : S.B + (size_t)n * S.ldb + k), v);
+        }
+        return v;
+    });
+    const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4, n = n0 + 4 * tx;
+    const bool stores = threadIdx.x < kTcThreads;
+    if (Gb.splits == 1) {
+        if (!stores) return;
+#pragma unroll 4
+        for (int r = ty; r < kTcM; r += kTcThreads / 16) gemm_finish(G, m0 + r, n, tile[r * kTcTileLd + tx]);
+        return;
+    }
+    // the blocks' partial tiles lie in their shared memories; each block finishes its share of the rows
+    cooperative_groups::cluster_group cluster = cooperative_groups::this_cluster();
+    cluster.sync();
+#pragma unroll 2
+    for (int r = kTcM * rank / Gb.splits + ty; stores && r < kTcM * (rank + 1) / Gb.splits; r += kTcThreads / 16) {
+        float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+        for (int k = 0; k < Gb.splits; k++) {
+            const float4 u = cluster.map_shared_rank(tile, k)[r * kTcTileLd + tx];
+            v.x += u.x; v.y += u.y; v.z += u.z; v.w += u.w;
+        }
+        gemm_finish(G, m0 + r, n, v);
+    }
+    cluster.sync();                                             // no block leaves while its tile is being read
 }
 
-// whether tc_gemm_kernel covers a batch: every N a multiple of the 128-wide tile, every K a multiple of 32
+// Whether the tensor cores take a batch: whole slices and tiles, enough rows, and a result that does not depend on how its
+// sums are formed.  Up to some 400 rows both kernels are one chain of latencies, and this one's is the longer (7.5 against
+// 7.1 us); at 600 rows and [128] -> [512] it takes 7.6 against 10.3.
+constexpr int kTcMinRows = 512;
 static bool tc_gemm_covers(const GemmBatch& Gb)
 {
+    if (Gb.whole || Gb.g[0].M < kTcMinRows) return false;
     for (int i = 0; i < Gb.n; i++) {
-        if (Gb.g[i].N % kTcTile) return false;
+        if (Gb.g[i].N % kTcN) return false;
         for (int s = 0; s < Gb.g[i].nseg; s++)
             if (Gb.g[i].seg[s].K % kTcKc) return false;
     }
     return true;
 }
 
-static int tc_gemm_batch(const GemmBatch& Gb, bool b_kn, cudaStream_t st)
+template <bool B_KN>
+static int launch_tc_gemm(GemmBatch& Gb, cudaStream_t st)
 {
     const GemmArgs& G = Gb.g[0];
-    static std::atomic<bool> attr_done[2][64];
+    auto kern = tc_gemm_kernel<B_KN>;
+    static std::atomic<bool> attr_done[64];
     int dev = 0;
     cudaGetDevice(&dev);
-    auto kern = b_kn ? tc_gemm_kernel<true> : tc_gemm_kernel<false>;
-    if (!attr_done[b_kn ? 1 : 0][dev & 63]) {
+    if (!attr_done[dev & 63]) {
         if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kTcSmemBytes) != cudaSuccess) return CFB200_E_CUDA;
-        attr_done[b_kn ? 1 : 0][dev & 63] = true;
+        attr_done[dev & 63] = true;
     }
-    const dim3 grid((G.M + kTcTile - 1) / kTcTile, G.N / kTcTile, Gb.n);
-    kern<<<grid, kTcThreads, kTcSmemBytes, st>>>(Gb);
-    return cudaGetLastError() == cudaSuccess ? CFB200_OK : CFB200_E_CUDA;
+    int slices = 0;
+    for (int s = 0; s < G.nseg; s++) slices += G.seg[s].K / kTcKc;
+    const unsigned gx = (unsigned)((G.M + kTcM - 1) / kTcM), gy = (unsigned)(G.N / kTcN);
+    // blocks that share a tile's contraction: as many as have four slices each, up to four, while all are resident at once
+    int splits = slices / 4 < 4 ? slices / 4 : 4;
+    while (splits > 1 && (int64_t)gx * gy * Gb.n * splits > 2 * (int64_t)sm_count()) splits--;
+    Gb.splits = splits < 1 ? 1 : splits;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(gx, gy, (unsigned)(Gb.n * Gb.splits));
+    cfg.blockDim = dim3(kTcBlock);
+    cfg.dynamicSmemBytes = kTcSmemBytes;
+    cfg.stream = st;
+    cudaLaunchAttribute attr = {};
+    attr.id = cudaLaunchAttributeClusterDimension;
+    attr.val.clusterDim.x = 1; attr.val.clusterDim.y = 1; attr.val.clusterDim.z = (unsigned)Gb.splits;
+    cfg.attrs = &attr;
+    cfg.numAttrs = Gb.splits > 1 ? 1 : 0;
+    return cudaLaunchKernelEx(&cfg, kern, (const GemmBatch)Gb) == cudaSuccess ? CFB200_OK : CFB200_E_CUDA;
+}
+
+static int tc_gemm_batch(GemmBatch& Gb, bool b_kn, cudaStream_t st)
+{
+    return b_kn ? launch_tc_gemm<true>(Gb, st) : launch_tc_gemm<false>(Gb, st);
 }
 
 // ---- weight gradients: out[P,Q] = A[M,P]^T B[M,Q], rows split over gridDim.y, partial tiles to scratch -------
-// Same problem table, scratch layout and reduction as wgrad_kernel (linear.cu); tiles are 128 x 128 and both
-// operands are staged transposed (the contraction index, the atom, is the slow index of A and B in memory).
-__global__ void __launch_bounds__(kTcThreads, 1) tc_wgrad_kernel(const WgArgs W)
+// Same problem table, scratch layout and reduction as wgrad_kernel (linear.cu); tiles are 128 x 64 and both operands are
+// staged transposed (the contraction index, the atom, is the slow index of A and B in memory).
+__global__ void __launch_bounds__(kTcBlock, 2) tc_wgrad_kernel(const WgArgs W)
 {
     extern __shared__ uint8_t tc_smem[];
-    __shared__ uint64_t mbar_slots[2];
+    __shared__ uint64_t mbar_slots[2 * kTcStages];
     __shared__ uint32_t tmem_slot;
     const int tid = threadIdx.x;
     int pi = 0;
     while (pi + 1 < W.nprob && (int)blockIdx.x >= W.prob[pi + 1].tile0) pi++;
     const WgProblem& Pb = W.prob[pi];
     const int t = blockIdx.x - Pb.tile0;
-    const int p0 = (t / Pb.tiles_q) * kTcTile, q0 = (t % Pb.tiles_q) * kTcTile;
+    const int p0 = (t / Pb.tiles_q) * kTcM, q0 = (t % Pb.tiles_q) * kTcN;
     const int split = blockIdx.y;
     const int r0 = split * W.rows, r1 = min(W.M, r0 + W.rows);
-    TcCta T;
-    tc_begin(T, tc_smem, mbar_slots, &tmem_slot);
-    TcOperand OA, OB;
-    OA.src = Pb.A; OA.ld = Pb.lda; OA.rows = Pb.P; OA.transposed = 1;
-    OB.src = Pb.B; OB.ld = Pb.ldb; OB.rows = Pb.Q; OB.transposed = 1;
+    const bool want_bias = Pb.bias_out != nullptr && q0 == 0;
     const int total = r1 > r0 ? (r1 - r0 + kTcKc - 1) / kTcKc : 0;
-    auto fetch = [&](TcSlice& R, int slice) {
-        if (slice >= total) return;
-        tc_fetch1(R.a, OA, p0, r0 + slice * kTcKc, r1, tid);
-        tc_fetch1(R.b, OB, q0, r0 + slice * kTcKc, r1, tid);
+    TcFetch<kTcM, true> FA;
+    TcFetch<kTcN, true> FB;
+    FA.open(Pb.A, Pb.lda, p0, Pb.P, r0, r1);
+    FB.open(Pb.B, Pb.ldb, q0, Pb.Q, r0, r1);
+    auto fetch = [&](TcSlice& R) { FA.next(R.a); FB.next(R.b); };       // rows beyond r1 read as zeros
+    float4 col = make_float4(0.f, 0.f, 0.f, 0.f);               // column sums of A over this thread's rows of the batch (the
+    static_assert(kTcThreads % (kTcM / 4) == 0, "");             // float4 of a thread lie in the same columns)
+    TcCta T;
+    auto step = [&](const TcSlice& R) {
+        if (want_bias) {
+#pragma unroll
+            for (int i = 0; i < tc_float4(kTcM); i++) { col.x += R.a[i].x; col.y += R.a[i].y; col.z += R.a[i].z; col.w += R.a[i].w; }
+        }
+        tc_slice<true, true>(T, R);
     };
-    TcSlice R0, R1, R2;
-    fetch(R0, 0); fetch(R1, 1); fetch(R2, 2);
-    for (int s = 0; s < total; s += 3) {
-        tc_slice(T, R0, OA, OB); fetch(R0, s + 3);
-        if (s + 1 < total) { tc_slice(T, R1, OA, OB); fetch(R1, s + 4); }
-        if (s + 2 < total) { tc_slice(T, R2, OA, OB); fetch(R2, s + 5); }
+    TcSlice R0, R1;
+    const bool brings = tid < kTcThreads;
+    if (brings) { fetch(R0); fetch(R1); }
+    tc_begin(T, tc_smem, mbar_slots, &tmem_slot);
+    if (brings) {
+        for (int s = 0; s < total; s += 2) {
+            step(R0); fetch(R0);
+            if (s + 1 < total) { step(R1); fetch(R1); }
+        }
+    } else if (tid == kTcThreads) {
+        tc_issue<true, true>(T, total);
     }
-    const bool have = tc_finish(T);
+    __syncwarp();
+    const float4* tile = tc_finish(T, total, [&](const int p, const int q) {
+        float v = 0.f;
+        for (int r = r0; r < r1; r++) v = fmaf(__ldg(Pb.A + (size_t)r * Pb.lda + p0 + p), __ldg(Pb.B + (size_t)r * Pb.ldb + q0 + q), v);
+        return v;
+    });
     float* ws = W.ws + Pb.ws_off + (size_t)split * Pb.P * Pb.Q;
-    const int p = p0 + tc_row();
-    for (int c0 = tc_col0(); c0 < tc_col0() + kTcTile / 2; c0 += 16) {
-        float v[16];
-        if (have) tc_load16(T.tmem, c0, v);
-        else {
+#pragma unroll 4
+    for (int r = tid >> 4; brings && r < kTcM; r += kTcThreads / 16)
+        *reinterpret_cast<float4*>(ws + (size_t)(p0 + r) * Pb.Q + q0 + 4 * (tid & 15)) = tile[r * kTcTileLd + (tid & 15)];
+    if (want_bias) {
+        // threads tid, tid + 32, ... hold the same columns: eight partial sums beside the tile
+        float4* part = const_cast<float4*>(tile) + kTcM * kTcTileLd;
+        if (brings) part[tid] = col;
+        __syncthreads();
+        if (tid < kTcM / 4) {
+            float4 v = part[tid];
 #pragma unroll
-            for (int i = 0; i < 16; i++) v[i] = 0.f;          // an empty row range contributes zeros
-        }
-        const int q = q0 + c0;
-        if ((have || total == 0) && p < Pb.P && q < Pb.Q) {
-#pragma unroll
-            for (int q4 = 0; q4 < 4; q4++)
-                *reinterpret_cast<float4*>(ws + (size_t)p * Pb.Q + q + 4 * q4) = make_float4(v[4 * q4], v[4 * q4 + 1], v[4 * q4 + 2], v[4 * q4 + 3]);
+            for (int w = 1; w < kTcThreads * 4 / kTcM; w++) { const float4 u = part[tid + w * (kTcM / 4)]; v.x += u.x; v.y += u.y; v.z += u.z; v.w += u.w; }
+            float* o = W.ws + Pb.ws_off + (size_t)W.S * Pb.P * Pb.Q + (size_t)split * Pb.P + p0 + 4 * tid;
+            o[0] = v.x; o[1] = v.y; o[2] = v.z; o[3] = v.w;
         }
     }
-    tc_end(T);
 }
 
-// Partial column sums of A (the bias gradients) for the problems that ask for them: grid (problem, split),
-// thread = column.  Same scratch slots as wgrad_kernel's.
-__global__ void __launch_bounds__(256) wgrad_colsum_kernel(const WgArgs W)
+// whether the tensor cores take a weight gradient: whole tiles, enough rows
+static bool tc_wgrad_covers(const WgProblem& Pb, int64_t M)
 {
-    const WgProblem& Pb = W.prob[blockIdx.x];
-    if (Pb.bias_out == nullptr) return;
-    const int split = blockIdx.y;
-    const int r0 = split * W.rows, r1 = min(W.M, r0 + W.rows);
-    for (int p = threadIdx.x; p < Pb.P; p += blockDim.x) {
-        float s = 0.f;
-        for (int r = r0; r < r1; r++) s += __ldg(Pb.A + (size_t)r * Pb.lda + p);
-        W.ws[Pb.ws_off + (size_t)W.S * Pb.nb * Pb.P * Pb.Q + (size_t)split * Pb.P + p] = s;
-    }
+    return M >= kTcMinRows && Pb.nb == 1 && Pb.P % kTcM == 0 && Pb.Q % kTcN == 0;
 }
 
 static int tc_wgrad_launch(const WgArgs& W, int tiles, cudaStream_t st)
@@ -401,8 +548,7 @@ static int tc_wgrad_launch(const WgArgs& W, int tiles, cudaStream_t st)
         if (cudaFuncSetAttribute(tc_wgrad_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kTcSmemBytes) != cudaSuccess) return CFB200_E_CUDA;
         attr_done[dev & 63] = true;
     }
-    tc_wgrad_kernel<<<dim3(tiles, W.S), kTcThreads, kTcSmemBytes, st>>>(W);
-    wgrad_colsum_kernel<<<dim3(W.nprob, W.S), 256, 0, st>>>(W);
+    tc_wgrad_kernel<<<dim3(tiles, W.S), kTcBlock, kTcSmemBytes, st>>>(W);
     return cudaGetLastError() == cudaSuccess ? CFB200_OK : CFB200_E_CUDA;
 }
 
