@@ -197,6 +197,117 @@ __device__ __forceinline__ float2 fw_project(const float* W_s, const float* rows
     return out;
 }
 
+// What a lane of the walk knows of the bases.  Windows, one byte per basis (distance, three axes): with lo the first index
+// inside, this lane's index l is inside when l >= lo and l <= lo + win - 1, and l + 32 when l + 32 >= lo and l + 32 <=
+// lo + win - 1.  Each comparison is bit 6 of a byte of a packed difference biased by 64 (no byte leaves 0..127), so that four
+// additions and two ANDs serve the four bases.
+struct FwLane {
+    unsigned in0_lo, in0_hi, in1_lo, in1_hi;
+    float cd_lo, cd_hi, nca_lo, nca_hi;      // basis constants, pre-scaled so that a Gaussian is ex2(-b*b)
+    float d0, dstep, a0, nastep;             // the same as number of the lane's first index, and step
+    bool wide_d;
+    __device__ __forceinline__ FwLane(const Params& P, const int lane)
+    {
+        const unsigned lane4 = lane * 0x01010101u;
+        const unsigned wins = (unsigned)P.win_dist | (unsigned)P.win_ang * 0x01010100u;
+        in0_lo = 0x40404040u + lane4; in0_hi = 0x3F3F3F3Fu + wins - lane4;
+        in1_lo = 0x60606060u + lane4; in1_hi = 0x1F1F1F1Fu + wins - lane4;
+        const float astep = P.a_step * kLlSqrtLog2e;
+        dstep = P.d_step * kLlSqrtLog2e; nastep = -astep;
+        d0 = (float)(lane + 1); a0 = (float)(P.angle_dim - 1 - lane);
+        cd_lo = (float)(lane + 1) * dstep; cd_hi = (float)(lane + 33) * dstep;
+        nca_lo = -(float)(P.angle_dim - 1 - lane) * astep; nca_hi = -(float)(P.angle_dim - 33 - lane) * astep;
+        wide_d = P.win_dist > 32;
+    }
+};
+
+// the record of a translation with weight exp(arg) relative to the pair's nearest, for (atom, head) ih; third: what the
+// walk multiplies its Gaussians with
+template <int AH>
+__device__ __forceinline__ void fw_record(const AtArgs& A, const Params& P, const int64_t ih, float* dst, const float arg, const float d2,
+                                          const float dx, const float dy, const float dz, const float third, const int flag)
+{
+    // d and 1/d from one reciprocal square root plus a Newton step; quotients by the basis spacings
+    // become products with their reciprocals (last-bit differences from IEEE sqrt / division)
+    float rinv = rsqrtf(fmaxf(d2, 1e-30f));
+    rinv = rinv * fmaf(-0.5f * d2 * rinv, rinv, 1.5f);
+    const float d = d2 * rinv;
+    int lo_d = 0;
+    if (P.windowed_dist) {
+        lo_d = (int)(fmaf(d, P.inv_d_interval, -P.d_cut_scaled) - 1.0f);
+        lo_d = min(max(lo_d, 0), 64 - P.win_dist);
+    }
+    float xa[3] = {0.f, 0.f, 0.f};
+    int lo_pack = lo_d;
+    if constexpr (AH > 0) {
+#pragma unroll
+        for (int x = 0; x < 3; x++) {
+            const float* F = A.frame[x] + ih * 3;
+            float cosv = 1e3f;
+            if (d2 > 1e-5f) cosv = fmaf(dz, __ldg(F + 2), fmaf(dy, __ldg(F + 1), dx * __ldg(F))) * rinv;
+            if (P.cos_abs) cosv = fabsf(cosv);
+            int lo = 0;
+            if (P.windowed_ang) {
+                const float en = fmaf(cosv + 1.0f + P.a_cut, P.inv_a_interval, 1.0f);
+                int end = (int)fminf(en, (float)P.angle_dim);
+                end = max(end, P.win_ang);
+                lo = end - P.win_ang;
+            }
+            xa[x] = (1.0f - cosv) * P.xa_scale;
+            lo_pack |= lo << (8 * (x + 1));
+        }
+    }
+    // minus the log2 of the weight
+    float4* o = reinterpret_cast<float4*>(dst);
+    o[0] = make_float4(-(arg * kLlLog2e), -d * P.xd_scale, third, __int_as_float(flag));
+    if constexpr (AH > 0) o[1] = make_float4(xa[0], xa[1], xa[2], __int_as_float(lo_pack));
+    else o[1].x = __int_as_float(lo_pack);
+}
+
+// lane = basis index: the Gaussians, times the weight, of record R (u its first half) that fall on this lane: add(k, value),
+// k as the lane numbers its indices (distance l, l + 32, axis 1 l, ...).  ONE_ROUNDING: a Gaussian's argument is the fused
+// x + number * step, as the compiler forms it in LatticeLane, and not x + (rounded constant).
+template <int AH, bool ONE_ROUNDING, class Add>
+__device__ __forceinline__ void fw_gaussians(const FwLane& L, const float4* R, const float4& u, Add&& add)
+{
+    const float nlw = u.x, xd = u.y;
+    float xa[3];
+    unsigned lo;
+    if constexpr (AH > 0) {
+        const float4 v = R[1];
+        xa[0] = v.x; xa[1] = v.y; xa[2] = v.z; lo = __float_as_uint(v.w);
+    } else {
+        lo = *reinterpret_cast<const unsigned*>(R + 1);
+    }
+    const unsigned in0 = (L.in0_lo - lo) & (L.in0_hi + lo), in1 = (L.in1_lo - lo) & (L.in1_hi + lo);
+    if (!L.wide_d) {                                        // at most one of the lane's two indices is in the window
+        const bool hi = in1 & 0x40u;
+        const float b = ONE_ROUNDING ? fmaf(hi ? L.d0 + 32.0f : L.d0, L.dstep, xd) : xd + (hi ? L.cd_hi : L.cd_lo);
+        const float g = ex2_approx(-fmaf(b, b, nlw));
+        if (in0 & 0x40u) add(0, g);
+        if (hi) add(1, g);
+    } else {
+        const float b0 = ONE_ROUNDING ? fmaf(L.d0, L.dstep, xd) : xd + L.cd_lo;
+        const float b1 = ONE_ROUNDING ? fmaf(L.d0 + 32.0f, L.dstep, xd) : xd + L.cd_hi;
+        const float g0 = ex2_approx(-fmaf(b0, b0, nlw)), g1 = ex2_approx(-fmaf(b1, b1, nlw));
+        if (in0 & 0x40u) add(0, g0);
+        if (in1 & 0x40u) add(1, g1);
+    }
+    if constexpr (AH > 0) {
+#pragma unroll
+        for (int x = 0; x < 3; x++) {
+            const float b0 = ONE_ROUNDING ? fmaf(L.a0, L.nastep, xa[x]) : xa[x] + L.nca_lo;
+            const float g0 = ex2_approx(-fmaf(b0, b0, nlw));
+            if (in0 & (0x4000u << (8 * x))) add(2 + AH * x, g0);
+            if constexpr (AH == 2) {
+                const float b1 = ONE_ROUNDING ? fmaf(L.a0 - 32.0f, L.nastep, xa[x]) : xa[x] + L.nca_hi;
+                const float g1 = ex2_approx(-fmaf(b1, b1, nlw));
+                if (in1 & (0x4000u << (8 * x))) add(3 + AH * x, g1);
+            }
+        }
+    }
+}
+
 template <int AH, bool TASKS, int MODE>
 __global__ void __launch_bounds__(fw_warps(MODE) * 32, fw_blocks(MODE)) attn_tile_kernel(const AtArgs A, const Params P)
 {
@@ -213,19 +324,7 @@ __global__ void __launch_bounds__(fw_warps(MODE) * 32, fw_blocks(MODE)) attn_til
     float* rows = W_s + kAtHd * K + kWarps * (32 * RS + 5 * kFwStage) + warp * fw_rows(MODE) * K;   // basis vectors to project: per basis
                                                             // (lane, half) pairs, or lanes where there is one half
     float2* wait = reinterpret_cast<float2*>(W_s + kAtHd * K + kWarps * (32 * RS + 5 * kFwStage)) + warp * kFwWait * kFwWaitLd;
-    // Windows, one byte per basis (distance, three axes): with lo the first index inside, this lane's index l is inside
-    // when l >= lo and l <= lo + win - 1, and l + 32 when l + 32 >= lo and l + 32 <= lo + win - 1.  Each comparison is bit
-    // 6 of a byte of a packed difference biased by 64 (no byte leaves 0..127), so that four additions and two ANDs
-    // serve the four bases.
-    const unsigned lane4 = lane * 0x01010101u;
-    const unsigned wins = (unsigned)P.win_dist | (unsigned)P.win_ang * 0x01010100u;
-    const unsigned in0_lo = 0x40404040u + lane4, in0_hi = 0x3F3F3F3Fu + wins - lane4;
-    const unsigned in1_lo = 0x60606060u + lane4, in1_hi = 0x1F1F1F1Fu + wins - lane4;
-    // per-lane basis constants, pre-scaled so that a Gaussian is ex2(-b*b)
-    const float dstep = P.d_step * kLlSqrtLog2e, astep = P.a_step * kLlSqrtLog2e;
-    const float cd_lo = (float)(lane + 1) * dstep, cd_hi = (float)(lane + 33) * dstep;
-    const float nca_lo = -(float)(P.angle_dim - 1 - lane) * astep, nca_hi = -(float)(P.angle_dim - 33 - lane) * astep;
-    const bool wide_d = P.win_dist > 32;
+    const FwLane L(P, lane);
     const float cut = fmaxf(P.prune, kFwCut);
     __shared__ int head_open;
 
@@ -410,42 +509,9 @@ __global__ void __launch_bounds__(fw_warps(MODE) * 32, fw_blocks(MODE)) attn_til
         // lane = translation: the record of a translation with weight exp(arg) relative to the pair's nearest
         auto make_record = [&](const int slot, const float arg, const float d2, const float dx, const float dy, const float dz,
                                const float fj, const int flag) {
-            // d and 1/d from one reciprocal square root plus a Newton step; quotients by the basis spacings
-            // become products with their reciprocals (last-bit differences from IEEE sqrt / division)
-            float rinv = rsqrtf(fmaxf(d2, 1e-30f));
-            rinv = rinv * fmaf(-0.5f * d2 * rinv, rinv, 1.5f);
-            const float d = d2 * rinv;
-            int lo_d = 0;
-            if (P.windowed_dist) {
-                lo_d = (int)(fmaf(d, P.inv_d_interval, -P.d_cut_scaled) - 1.0f);
-                lo_d = min(max(lo_d, 0), 64 - P.win_dist);
-            }
-            float xa[3] = {0.f, 0.f, 0.f};
-            int lo_pack = lo_d;
-            if constexpr (AH > 0) {
-#pragma unroll
-                for (int x = 0; x < 3; x++) {
-                    const float* F = A.frame[x] + ih * 3;
-                    float cosv = 1e3f;
-                    if (d2 > 1e-5f) cosv = fmaf(dz, __ldg(F + 2), fmaf(dy, __ldg(F + 1), dx * __ldg(F))) * rinv;
-                    if (P.cos_abs) cosv = fabsf(cosv);
-                    int lo = 0;
-                    if (P.windowed_ang) {
-                        const float en = fmaf(cosv + 1.0f + P.a_cut, P.inv_a_interval, 1.0f);
-                        int end = (int)fminf(en, (float)P.angle_dim);
-                        end = max(end, P.win_ang);
-                        lo = end - P.win_ang;
-                    }
-                    xa[x] = (1.0f - cosv) * P.xa_scale;
-                    lo_pack |= lo << (8 * (x + 1));
-                }
-            }
-            // minus the log2 of the weight; forward the soft-max weight (d^2 where a pair's sums are kept), backward
-            // d^2 less the nearest one's (fj), which keeps t_ij - x_ij s_ij from cancelling
-            float4* o = reinterpret_cast<float4*>(rec + slot * RS);
-            o[0] = make_float4(-(arg * kLlLog2e), -d * P.xd_scale, BACK ? d2 - fj : (SAVE ? d2 : fj), __int_as_float(flag));
-            if constexpr (AH > 0) o[1] = make_float4(xa[0], xa[1], xa[2], __int_as_float(lo_pack));
-            else o[1].x = __int_as_float(lo_pack);
+            // third: the soft-max weight forward (d^2 where a pair's sums are kept); d^2 less the nearest one's (fj) backward,
+            // which keeps t_ij - x_ij s_ij from cancelling
+            fw_record<AH>(A, P, ih, rec + slot * RS, arg, d2, dx, dy, dz, BACK ? d2 - fj : (SAVE ? d2 : fj), flag);
         };
 
         // lane = basis index: the walk over n records
@@ -453,48 +519,14 @@ __global__ void __launch_bounds__(fw_warps(MODE) * 32, fw_blocks(MODE)) attn_til
             const float4* R = reinterpret_cast<const float4*>(rec);
             for (int r = 0; r < n; r++, R += RS / 4) {
                 const float4 u = R[0];
-                const float nlw = u.x, xd = u.y, fw = u.z;
+                const float fw = u.z;
                 const int flag = __float_as_int(u.w);
-                float xa[3];
-                unsigned lo;
-                if constexpr (AH > 0) {
-                    const float4 v = R[1];
-                    xa[0] = v.x; xa[1] = v.y; xa[2] = v.z; lo = __float_as_uint(v.w);
-                } else {
-                    lo = *reinterpret_cast<const unsigned*>(R + 1);
-                }
-                const unsigned in0 = (in0_lo - lo) & (in0_hi + lo), in1 = (in1_lo - lo) & (in1_hi + lo);
                 float u_back = 0.f;
-                auto add = [&](const int k, const float g) {
+                fw_gaussians<AH, false>(L, R, u, [&](const int k, const float g) {
                     if constexpr (BACK) u_back = fmaf(g, S[k], u_back);
                     else if constexpr (SAVE) { s[k] += g; T[k] = fmaf(g, fw, T[k]); }
                     else s[k] = fmaf(g, fw, s[k]);
-                };
-                if (!wide_d) {                              // at most one of the lane's two indices is in the window
-                    const bool hi = in1 & 0x40u;
-                    const float b = xd + (hi ? cd_hi : cd_lo);
-                    const float g = ex2_approx(-fmaf(b, b, nlw));
-                    if (in0 & 0x40u) add(0, g);
-                    if (hi) add(1, g);
-                } else {
-                    const float b0 = xd + cd_lo, b1 = xd + cd_hi;
-                    const float g0 = ex2_approx(-fmaf(b0, b0, nlw)), g1 = ex2_approx(-fmaf(b1, b1, nlw));
-                    if (in0 & 0x40u) add(0, g0);
-                    if (in1 & 0x40u) add(1, g1);
-                }
-                if constexpr (AH > 0) {
-#pragma unroll
-                    for (int x = 0; x < 3; x++) {
-                        const float b0 = xa[x] + nca_lo;
-                        const float g0 = ex2_approx(-fmaf(b0, b0, nlw));
-                        if (in0 & (0x4000u << (8 * x))) add(2 + AH * x, g0);
-                        if constexpr (AH == 2) {
-                            const float b1 = xa[x] + nca_hi;
-                            const float g1 = ex2_approx(-fmaf(b1, b1, nlw));
-                            if (in1 & (0x4000u << (8 * x))) add(3 + AH * x, g1);
-                        }
-                    }
-                }
+                });
                 if constexpr (BACK) { accB += u_back; accA = fmaf(u_back, fw, accA); }
                 if (MODE != 0 && flag) flush(flag - 1);
             }
@@ -575,10 +607,10 @@ __global__ void __launch_bounds__(fw_warps(MODE) * 32, fw_blocks(MODE)) attn_til
             float sum_lost = 0.f, px_lost = 0.f;            // what the additions below rounded away
             int cnt = 0;
             if (use_list) {
-                const float* L1 = A.list + (size_t)(on ? e : e0) * kListStride;
+                const float* Lq = A.list + (size_t)(on ? e : e0) * kListStride;
                 auto quad = [&](const int q) {
-                    if (A.vec_list) return __ldg(reinterpret_cast<const float4*>(L1) + q);
-                    return make_float4(__ldg(L1 + 4 * q), __ldg(L1 + 4 * q + 1), __ldg(L1 + 4 * q + 2), __ldg(L1 + 4 * q + 3));
+                    if (A.vec_list) return __ldg(reinterpret_cast<const float4*>(Lq) + q);
+                    return make_float4(__ldg(Lq + 4 * q), __ldg(Lq + 4 * q + 1), __ldg(Lq + 4 * q + 2), __ldg(Lq + 4 * q + 3));
                 };
                 float4 u = quad(0);
                 ref = u.x;
@@ -819,8 +851,9 @@ __global__ void __launch_bounds__(fw_warps(MODE) * 32, fw_blocks(MODE)) attn_til
 // itself, an online soft-max over the pairs; leaves per-pair results.  Same results as attn_tile_kernel to rounding.  Bound by
 // instruction issue: 800 per (pair, head) in cells of 100-200 atoms, nearly all of them fixed.  Two uses:
 // * batches without translation lists, where the tiles are no faster (see attn_fused_fwd);
-// * the training forward of models with weighted-PCA frames, for its rounding (a training step of 16 crystals of 100-200
-//   atoms 17.5 ms with it, 8.2 with the tiles).  An eigenvector of the second moments has a sign and, where eigenvalues are
+// * the training forward of models with weighted-PCA frames, for its rounding: attn_ordered_kernel forms the same sums in
+//   tiles, and takes this way where a task's range has no list (a training step of 16 crystals of 100-200 atoms 16.8 ms with
+//   this kernel, 12.4 with that one, 8.2 with attn_tile_kernel).  An eigenvector of the second moments has a sign and, where eigenvalues are
 //   close, a direction that a last bit decides, and the ReLUs behind it turn with it.  In a batch whose errors have balanced
 //   signs the mean gradient is small, and one turned ReLU is then a quarter of its root mean square: of 150 batches of 16
 //   such crystals two moved by more than a tenth when the tiles' order of summation took the place of this one, while the
@@ -875,11 +908,13 @@ constexpr size_t kPwSmem = sizeof(float) * (kAtHd * kPwStride + kPwWarps * 8 * 3
 
 // out_d = W_d . row: lane = (output d, half of the 256 basis indices); every lane returns the full sum of its d.
 // Packed FP32: two products per instruction, two partial sums.
+// LD: floats between rows of W; GAP: floats between the halves of a row, of W and of the vector.
+template <int LD, int GAP>
 __device__ __forceinline__ float project_row(const float* W_s, const float* row, const int lane)
 {
     const int d = lane & 15, half = lane >> 4;
-    const ulonglong2* wr = reinterpret_cast<const ulonglong2*>(W_s + d * kPwStride) + half * 32;
-    const ulonglong2* sr = reinterpret_cast<const ulonglong2*>(row) + half * 32;
+    const ulonglong2* wr = reinterpret_cast<const ulonglong2*>(W_s + d * LD) + half * (32 + GAP / 4);
+    const ulonglong2* sr = reinterpret_cast<const ulonglong2*>(row) + half * (32 + GAP / 4);
     f32x2 acc = pack2(0.f, 0.f);
 #pragma unroll 8
     for (int k4 = 0; k4 < 32; k4++) {
@@ -891,6 +926,93 @@ __device__ __forceinline__ float project_row(const float* W_s, const float* row,
     unpack2(acc, a0, a1);
     const float sum = a0 + a1;
     return sum + __shfl_xor_sync(0xffffffffu, sum, 16);
+}
+
+// One task, its pairs one after the other.  srow: 3 x 256 + GAP floats of the warp's (the basis vector being projected, the pooled
+// sums plain and d^2-weighted); results go to row `row` (numbered from N: partial rows).
+template <bool ANG, int LD, int GAP>
+__device__ __forceinline__ void pairwise_task(const AtArgs& A, const Params& P, LatticeLane<2, ANG>& L, const AtomTask& T, int64_t row,
+                                              const bool partial, const int h, const float* W_s, float* srow, const int lane)
+{
+    const int H = P.H;
+    const int64_t i = T.i;
+    // pooled basis sums of this lane as four packed pairs (indices l, l + 32 of each basis): Sp[32 x], x < 4; then the
+    // d^2-weighted ones
+    f32x2* Sp = reinterpret_cast<f32x2*>(srow + kAtK + GAP) + lane;
+    f32x2* Tq = Sp + kAtK / 2;
+    const float qd = lane < kAtHd ? __ldg(A.qs + (i * H + h) * kAtHd + lane) : 0.f;
+    float m = -INFINITY, l = 0.f, V = 0.f;
+#pragma unroll
+    for (int x = 0; x < 4; x++) Sp[32 * x] = Tq[32 * x] = pack2(0.f, 0.f);        // attention-pooled sums, plain and d^2-weighted
+    const int64_t j0 = T.e1 > T.e0 ? A.edges[A.E + T.e0] : 0;
+    for (int64_t e = T.e0; e < T.e1; e++) {
+        const int64_t j = j0 + (e - T.e0);
+        if (lane == 0 && __ldg(A.edges + A.E + e) != j) atomicOr(&g_status, CFB200_ST_PAIR_LAYOUT);   // not the dense layout
+        float kd = 0.f, vd = 0.f;
+        if (lane < kAtHd) { kd = __ldg(A.k + (j * H + h) * kAtHd + lane); vd = __ldg(A.v + (j * H + h) * kAtHd + lane); }
+        run_pair(A, P, L, T, e);
+        float r0 = L.sum_l, r1 = L.px_l, r2 = qd * kd;
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) {
+            r0 += __shfl_xor_sync(0xffffffffu, r0, o); r1 += __shfl_xor_sync(0xffffffffu, r1, o);
+            r2 += __shfl_xor_sync(0xffffffffu, r2, o);
+        }
+        const float sum = r0, qk = r2;
+        const float inv = 1.0f / sum;
+        const float zv = logf(sum) + L.ref * L.a;
+        if (lane == 0) { A.z[e * H + h] = zv; A.px[e * H + h] = r1 * inv; }
+        // the pair's value encoding: its normalised basis sums, with the scaling of the values, times W
+        {
+            const float cd = inv * P.c_dist, ca = inv * P.c_ang;
+            srow[lane] = L.sd[0] * cd; srow[32 + lane] = L.sd[1] * cd;
+#pragma unroll
+            for (int x = 0; x < 3; x++) { srow[64 + 64 * x + (x > 0 ? GAP : 0) + lane] = L.sa[x][0] * ca; srow[96 + 64 * x + (x > 0 ? GAP : 0) + lane] = L.sa[x][1] * ca; }
+        }
+        __syncwarp();
+        const float val_d = project_row<LD, GAP>(W_s, srow, lane);
+        if (lane < kAtHd) A.val[(e * H + h) * kAtHd + lane] = val_d;
+        __syncwarp();
+        const float s = qk + zv;
+        const float mn = fmaxf(m, s);
+        const float sc = __expf(m - mn), p = __expf(s - mn);
+        const float f = p * inv;
+        l = fmaf(l, sc, p);
+        V = fmaf(V, sc, p * (vd + val_d));
+        {
+            const f32x2 sc2 = pack2(sc, sc), f2 = pack2(f, f);
+            Sp[0] = fma2(Sp[0], sc2, mul2(f2, pack2(L.sd[0], L.sd[1])));
+            Tq[0] = fma2(Tq[0], sc2, mul2(f2, pack2(L.qd[0], L.qd[1])));
+#pragma unroll
+            for (int x = 0; x < 3; x++) {
+                Sp[32 + 32 * x] = fma2(Sp[32 + 32 * x], sc2, mul2(f2, pack2(L.sa[x][0], L.sa[x][1])));
+                Tq[32 + 32 * x] = fma2(Tq[32 + 32 * x], sc2, mul2(f2, pack2(L.qa[x][0], L.qa[x][1])));
+            }
+        }
+        m = mn;
+    }
+    const float inv_l = T.e1 > T.e0 ? 1.0f / l : 0.f;
+    if (partial) row -= A.N;
+    if (lane == 0) (partial ? A.part_lse : A.lse)[row * H + h] = m + logf(l);
+    float* sp = (partial ? A.part_spool : A.spool) + (row * H + h) * kAtK;
+    {
+        float s0, s1, t0, t1;
+        unpack2(Sp[0], s0, s1); unpack2(Tq[0], t0, t1);
+        sp[lane] = s0 * inv_l; sp[32 + lane] = s1 * inv_l;
+        srow[lane] = t0 * inv_l * P.c_dist; srow[32 + lane] = t1 * inv_l * P.c_dist;
+#pragma unroll
+        for (int x = 0; x < 3; x++) {
+            unpack2(Sp[32 + 32 * x], s0, s1); unpack2(Tq[32 + 32 * x], t0, t1);
+            sp[64 + 64 * x + lane] = s0 * inv_l * P.c_ang; sp[96 + 64 * x + lane] = s1 * inv_l * P.c_ang;
+            srow[64 + 64 * x + (x > 0 ? GAP : 0) + lane] = t0 * inv_l * P.c_ang; srow[96 + 64 * x + (x > 0 ? GAP : 0) + lane] = t1 * inv_l * P.c_ang;
+        }
+    }
+    __syncwarp();
+    const float up_d = project_row<LD, GAP>(W_s, srow, lane);     // W (pooled d^2-weighted sums)
+    if (lane < kAtHd) {
+        (partial ? A.part_out : A.out)[(row * H + h) * kAtHd + lane] = V * inv_l;
+        (partial ? A.part_upool : A.upool)[(row * H + h) * kAtHd + lane] = up_d;
+    }
+    __syncwarp();
 }
 
 template <bool ANG, bool TASKS>
@@ -905,10 +1027,6 @@ __global__ void __launch_bounds__(kPwWarps * 32, 2) attn_pairwise_kernel(const A
     LatticeLane<2, ANG> L;
     L.init(P, lane, tbuf + warp * 8 * 32);
     float* srow = rows + warp * 3 * kAtK;
-    // pooled basis sums of this lane as four packed pairs (indices l, l + 32 of each basis): Sp[32 x], x < 4; then the
-    // d^2-weighted ones
-    f32x2* Sp = reinterpret_cast<f32x2*>(srow + kAtK) + lane;
-    f32x2* Tq = Sp + kAtK / 2;
     __shared__ int head_open;
 
     // heads in turn, as in attn_tile_kernel
@@ -960,78 +1078,333 @@ __global__ void __launch_bounds__(kPwWarps * 32, 2) attn_pairwise_kernel(const A
             row = i;
             T = load_atom(A, P, L, i, h, lane);
         }
-        const float qd = lane < kAtHd ? __ldg(A.qs + (i * H + h) * kAtHd + lane) : 0.f;
+        pairwise_task<ANG, kPwStride, 0>(A, P, L, T, row, TASKS && row >= A.N, h, W_s, srow, lane);
+    }
+    }   // heads in turn
+}
+
+// ---- the same sums in tiles ---------------------------------------------------------------------------------------
+// The forward one pair after the other, for tasks whose ranges have lists, with lanes used as in attn_tile_kernel and every
+// sum formed in the order of pairwise_task, so that each result is the same to the bit:
+//   * normaliser and mean d^2: lane = translation, four of the 125 per lane, then the tree of a butterfly over the lanes --
+//     walked for eight pairs at once, lane = (pair, quarter of the tree's leaves);
+//   * lane = pair: q.k as the butterfly adds its 16 products, logarithm, bias; the running maximum is a prefix maximum, and
+//     with it every factor of the online soft-max is known before the walk;
+//   * lane = translation: records; lane = basis index: the walk, which meets a pair's translations in the same order;
+//   * projection of four pairs at once: a lane runs the chains of two outputs and two pairs over half of the indices.
+// Bound by shared memory (the projection's reads: 133 wavefronts per pair and head, 60 % of the data path; 1.82 ms before its
+// rows were kept in different banks) and issue (490 instructions instead of 803, 55 % of the slots).  16 crystals of 100-200
+// atoms (2.7 M pairs and heads), per launch 2.65 -> 1.70 ms; a training step 16.8 -> 12.4 ms.
+constexpr int kOrWarps = 10;
+constexpr int kOrWait = 36;            // stride of the waiting partial sums: conflict-free 64-bit reads by (pair, quarter)
+// A row is two halves 16 banks apart, and two rows are 8 banks apart: the four addresses that a warp reads a row or W at meet
+// in as few banks as they can.
+constexpr int kOrGap = 16, kOrRow = 2 * 128 + kOrGap + 4;
+constexpr int kOrWarpFloats = 4 * kOrRow + 32 * kFwRec + 8 * kOrWait * 2 + 32 * 4;
+constexpr size_t kOrSmem = sizeof(float) * (kAtHd * kOrRow + kOrWarps * kOrWarpFloats);
+
+// tasks whose ranges have no list; not inlined, so that its registers are not the kernel's
+template <bool TASKS>
+__device__ __noinline__ void ordered_slow_task(const AtArgs& A, const Params& P, const int i, const int off, const int np, const int64_t row,
+                                               const int h, const float* W_s, float* warp_s)
+{
+    const int lane = threadIdx.x & 31;
+    LatticeLane<2, true> L;
+    L.init(P, lane, warp_s + 3 * kAtK + kOrGap);
+    AtomTask T = load_atom(A, P, L, i, h, lane);
+    T.e0 += off; T.e1 = T.e0 + np;
+    pairwise_task<true, kOrRow, kOrGap>(A, P, L, T, row, TASKS && row >= A.N, h, W_s, warp_s, lane);
+}
+
+template <bool TASKS>
+__global__ void __launch_bounds__(kOrWarps * 32, 2) attn_ordered_kernel(const __grid_constant__ AtArgs A, const __grid_constant__ Params P)
+{
+    extern __shared__ __align__(16) float smem[];
+    float* W_s = smem;                                      // [16][kOrRow]
+    const int H = P.H;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    float* rows = W_s + kAtHd * kOrRow + warp * kOrWarpFloats;           // four basis vectors being projected
+    float* rec = rows + 4 * kOrRow;
+    float2* wait = reinterpret_cast<float2*>(rec + 32 * kFwRec);            // [8][kOrWait]: lanes' parts of normaliser and sum w d^2
+    float4* pairs = reinterpret_cast<float4*>(rec + 32 * kFwRec + 8 * kOrWait * 2);    // per pair of the tile: sc, p, f, 1 / sum
+    const FwLane L(P, lane);
+    const bool vec = A.vec;
+    __shared__ int head_open;
+
+    // heads in turn, as in attn_tile_kernel
+    for (int turn = 0; turn < 2 * H; turn++) {
+    int h = blockIdx.y;
+    if (turn > 0) {
+        __syncthreads();                                    // every warp is done with the previous head's weights
+        if (threadIdx.x == 0) {
+            int best = -1, most = 0;
+            for (int hh = 0; hh < H; hh++) {
+                const int limit = TASKS ? (int)(A.n_entries - kSplitSlots) + __ldg(A.chunk_count + hh) : (int)A.N;
+                const int left = limit - atomicAdd(A.counters + hh, 0);
+                if (left > most) { most = left; best = hh; }
+            }
+            head_open = best;
+        }
+        __syncthreads();
+        h = head_open;
+        if (h < 0) break;                                   // every queue is drained
+    }
+    const int first = TASKS ? kSplitSlots - __ldg(A.chunk_count + h) : 0;
+    for (int idx = threadIdx.x; idx < kAtHd * kAtK; idx += kOrWarps * 32) {
+        const int o = idx >> 8, b = (idx >> 6) & 3, d = idx & 63;
+        const int width = b == 0 ? 64 : P.angle_dim;        // columns this basis' weights hold (zero beyond)
+        W_s[o * kOrRow + (idx & 255) + (b > 1 ? kOrGap : 0)] = d < width ? __ldg(A.W[b] + ((size_t)h * kAtHd + o) * width + d) : 0.f;
+    }
+    __syncthreads();
+
+    for (;;) {
+        const int64_t t = next_task(A.counters + h, lane) + first;
+        if (t >= (TASKS ? A.n_entries : A.N)) break;
+        int i, row, off = 0, np;
+        int64_t e0;
+        if (TASKS) {
+            const int4 d = __ldg(A.tasks + (size_t)h * A.n_entries + t);
+            np = d.w & 0xFFFFFF;
+            if (np == 0) continue;
+            i = d.x; row = d.y; off = d.z;
+            e0 = A.e_start[i];
+        } else {
+            i = A.order != nullptr ? A.order[t] : (int)t;
+            row = i;
+            e0 = A.e_start[i];
+            np = (int)(A.e_start[i + 1] - e0);
+        }
+        const int64_t ih = (int64_t)i * H + h;
+        const float a = __ldg(A.a_ik + ih);
+        int Rl = A.cache_range;
+        if (lane < 3) Rl = lattice_range_1d(P, a, P.cutoff_radius != 0.0f ? __ldg(A.rvlen + 3 * A.batch[i] + lane) : 0.0f);
+        if (__any_sync(0xffffffffu, Rl != A.cache_range)) {
+            ordered_slow_task<TASKS>(A, P, i, off, np, row, h, W_s, rows);
+            continue;
+        }
+        e0 += off;
+        const int j0 = np > 0 ? (int)A.edges[A.E + e0] : 0;
         float m = -INFINITY, l = 0.f, V = 0.f;
+        float s[8], T[8];                                   // the pair's sums, plain and d^2-weighted
+        f32x2 S[4], Tq[4];                                  // both pooled
 #pragma unroll
-        for (int x = 0; x < 4; x++) Sp[32 * x] = Tq[32 * x] = pack2(0.f, 0.f);        // attention-pooled sums, plain and d^2-weighted
-        const int64_t j0 = T.e1 > T.e0 ? A.edges[A.E + T.e0] : 0;
-        for (int64_t e = T.e0; e < T.e1; e++) {
-            const int64_t j = j0 + (e - T.e0);
-            if (lane == 0 && __ldg(A.edges + A.E + e) != j) atomicOr(&g_status, CFB200_ST_PAIR_LAYOUT);   // not the dense layout
-            float kd = 0.f, vd = 0.f;
-            if (lane < kAtHd) { kd = __ldg(A.k + (j * H + h) * kAtHd + lane); vd = __ldg(A.v + (j * H + h) * kAtHd + lane); }
-            run_pair(A, P, L, T, e);
-            float r0 = L.sum_l, r1 = L.px_l, r2 = qd * kd;
+        for (int r = 0; r < 8; r++) s[r] = T[r] = 0.f;
 #pragma unroll
-            for (int o = 16; o > 0; o >>= 1) {
-                r0 += __shfl_xor_sync(0xffffffffu, r0, o); r1 += __shfl_xor_sync(0xffffffffu, r1, o);
-                r2 += __shfl_xor_sync(0xffffffffu, r2, o);
-            }
-            const float sum = r0, qk = r2;
-            const float inv = 1.0f / sum;
-            const float zv = logf(sum) + L.ref * L.a;
-            if (lane == 0) { A.z[e * H + h] = zv; A.px[e * H + h] = r1 * inv; }
-            // the pair's value encoding: its normalised basis sums, with the scaling of the values, times W
+        for (int x = 0; x < 4; x++) S[x] = Tq[x] = pack2(0.f, 0.f);
+        int tile0 = 0;
+
+        auto flush = [&](const int j) {
+            const float4 pr = pairs[j];                     // sc, p, f, 1 / sum
             {
-                const float cd = inv * P.c_dist, ca = inv * P.c_ang;
-                srow[lane] = L.sd[0] * cd; srow[32 + lane] = L.sd[1] * cd;
+                const float cd = pr.w * P.c_dist, ca = pr.w * P.c_ang;
+                float* w = rows + (j & 3) * kOrRow + lane;
+                w[0] = s[0] * cd; w[32] = s[1] * cd;
 #pragma unroll
-                for (int x = 0; x < 3; x++) { srow[64 + 64 * x + lane] = L.sa[x][0] * ca; srow[96 + 64 * x + lane] = L.sa[x][1] * ca; }
-            }
-            __syncwarp();
-            const float val_d = project_row(W_s, srow, lane);
-            if (lane < kAtHd) A.val[(e * H + h) * kAtHd + lane] = val_d;
-            __syncwarp();
-            const float s = qk + zv;
-            const float mn = fmaxf(m, s);
-            const float sc = __expf(m - mn), p = __expf(s - mn);
-            const float f = p * inv;
-            l = fmaf(l, sc, p);
-            V = fmaf(V, sc, p * (vd + val_d));
-            {
-                const f32x2 sc2 = pack2(sc, sc), f2 = pack2(f, f);
-                Sp[0] = fma2(Sp[0], sc2, mul2(f2, pack2(L.sd[0], L.sd[1])));
-                Tq[0] = fma2(Tq[0], sc2, mul2(f2, pack2(L.qd[0], L.qd[1])));
-#pragma unroll
-                for (int x = 0; x < 3; x++) {
-                    Sp[32 + 32 * x] = fma2(Sp[32 + 32 * x], sc2, mul2(f2, pack2(L.sa[x][0], L.sa[x][1])));
-                    Tq[32 + 32 * x] = fma2(Tq[32 + 32 * x], sc2, mul2(f2, pack2(L.qa[x][0], L.qa[x][1])));
+                for (int x = 1; x < 4; x++) {
+                    const int at = 64 * x + (x > 1 ? kOrGap : 0);
+                    w[at] = s[2 * x] * ca; w[at + 32] = s[2 * x + 1] * ca;
                 }
             }
-            m = mn;
-        }
-        const float inv_l = T.e1 > T.e0 ? 1.0f / l : 0.f;
-        const bool partial = TASKS && row >= A.N;
-        if (partial) row -= A.N;
-        if (lane == 0) (partial ? A.part_lse : A.lse)[row * H + h] = m + logf(l);
-        float* sp = (partial ? A.part_spool : A.spool) + (row * H + h) * kAtK;
-        {
-            float s0, s1, t0, t1;
-            unpack2(Sp[0], s0, s1); unpack2(Tq[0], t0, t1);
-            sp[lane] = s0 * inv_l; sp[32 + lane] = s1 * inv_l;
-            srow[lane] = t0 * inv_l * P.c_dist; srow[32 + lane] = t1 * inv_l * P.c_dist;
+            l = fmaf(l, pr.x, pr.y);
+            const f32x2 sc2 = pack2(pr.x, pr.x), f2 = pack2(pr.z, pr.z);
 #pragma unroll
-            for (int x = 0; x < 3; x++) {
-                unpack2(Sp[32 + 32 * x], s0, s1); unpack2(Tq[32 + 32 * x], t0, t1);
-                sp[64 + 64 * x + lane] = s0 * inv_l * P.c_ang; sp[96 + 64 * x + lane] = s1 * inv_l * P.c_ang;
-                srow[64 + 64 * x + lane] = t0 * inv_l * P.c_ang; srow[96 + 64 * x + lane] = t1 * inv_l * P.c_ang;
+            for (int x = 0; x < 4; x++) {
+                S[x] = fma2(S[x], sc2, mul2(f2, pack2(s[2 * x], s[2 * x + 1])));
+                Tq[x] = fma2(Tq[x], sc2, mul2(f2, pack2(T[2 * x], T[2 * x + 1])));
+            }
+#pragma unroll
+            for (int r = 0; r < 8; r++) s[r] = T[r] = 0.f;
+            if ((j & 3) != 3 && tile0 + j != np - 1) return;
+            // value encodings of up to four pairs: lane = (half of the indices, pair of pairs, outputs o and o + 8)
+            const int n = (j & 3) + 1, o = lane & 7, rp = (lane >> 3) & 1, half = lane >> 4;
+            const int64_t ef = e0 + tile0 + (j & ~3);
+            const float* vp = A.v + ((int64_t)(j0 + tile0 + (j & ~3)) * H + h) * kAtHd + (lane & 15);
+            float vd[4];
+#pragma unroll
+            for (int r = 0; r < 4; r++) vd[r] = r < n ? __ldg(vp + (int64_t)r * H * kAtHd) : 0.f;
+            __syncwarp();
+            const ulonglong2* w0 = reinterpret_cast<const ulonglong2*>(W_s + o * kOrRow) + half * (32 + kOrGap / 4);
+            const ulonglong2* w1 = w0 + 8 * kOrRow / 4;
+            const ulonglong2* r0 = reinterpret_cast<const ulonglong2*>(rows + 2 * rp * kOrRow) + half * (32 + kOrGap / 4);
+            const ulonglong2* r1 = r0 + kOrRow / 4;
+            f32x2 acc[2][2];
+            acc[0][0] = acc[0][1] = acc[1][0] = acc[1][1] = pack2(0.f, 0.f);
+#pragma unroll 4
+            for (int k = 0; k < 32; k++) {
+                const ulonglong2 wa = w0[k], wb = w1[k], ra = r0[k], rb = r1[k];
+                acc[0][0] = fma2(ra.x, wa.x, acc[0][0]); acc[0][0] = fma2(ra.y, wa.y, acc[0][0]);
+                acc[0][1] = fma2(ra.x, wb.x, acc[0][1]); acc[0][1] = fma2(ra.y, wb.y, acc[0][1]);
+                acc[1][0] = fma2(rb.x, wa.x, acc[1][0]); acc[1][0] = fma2(rb.y, wa.y, acc[1][0]);
+                acc[1][1] = fma2(rb.x, wb.x, acc[1][1]); acc[1][1] = fma2(rb.y, wb.y, acc[1][1]);
+            }
+            float q[2];                                     // this lane passes on output o + 8 half of its two pairs
+#pragma unroll
+            for (int r = 0; r < 2; r++) {
+                float x, y, v[2];
+                unpack2(acc[r][0], x, y);
+                v[0] = x + y;
+                unpack2(acc[r][1], x, y);
+                v[1] = x + y;
+#pragma unroll
+                for (int c = 0; c < 2; c++) v[c] = v[c] + __shfl_xor_sync(0xffffffffu, v[c], 16);
+                q[r] = half ? v[1] : v[0];
+                if (2 * rp + r < n) A.val[((ef + 2 * rp + r) * H + h) * kAtHd + o + 8 * half] = q[r];
+            }
+#pragma unroll
+            for (int r = 0; r < 4; r++) {
+                const float val_d = __shfl_sync(0xffffffffu, q[r & 1], ((lane & 8) << 1) + (r >> 1) * 8 + (lane & 7));
+                if (r < n) {
+                    const float4 pv = pairs[(j & ~3) + r];
+                    V = fmaf(V, pv.x, pv.y * (vd[r] + val_d));
+                }
+            }
+            __syncwarp();
+        };
+
+        for (tile0 = 0; tile0 < np; tile0 += 32) {
+            const int nt = min(32, np - tile0);
+            const bool on = lane < nt;
+            const int64_t e = e0 + tile0 + lane, j = (int64_t)j0 + tile0 + lane;
+            // ---- lane = translation: normalisers, eight pairs at a time ----
+            float sum = 1.f, px = 0.f;
+            int cnt = 0;
+            for (int g = 0; g < nt; g += 8) {
+                const int n = min(8, nt - g);
+                const float* Ll = A.list + (size_t)(e0 + tile0 + g) * kListStride + lane;
+#pragma unroll 4
+                for (int k = 0; k < n; k++, Ll += kListStride) {
+                    const float d0 = __ldg(Ll), d1 = __ldg(Ll + 32), d2 = __ldg(Ll + 64), d3 = __ldg(Ll + 96);
+                    const float ref = __shfl_sync(0xffffffffu, d0, 0);
+                    const float a0 = a * (d0 - ref), a1 = a * (d1 - ref), a2 = a * (d2 - ref), a3 = a * (d3 - ref);
+                    const float w0 = ex2_approx(a0 * kLlLog2e), w1 = ex2_approx(a1 * kLlLog2e), w2 = ex2_approx(a2 * kLlLog2e),
+                                w3 = ex2_approx(a3 * kLlLog2e);
+                    wait[k * kOrWait + lane] = make_float2(((w0 + w1) + w2) + w3, fmaf(w3, d3, fmaf(w2, d2, fmaf(w1, d1, w0 * d0))));
+                    int c = __popc(__ballot_sync(0xffffffffu, a0 > -P.prune));
+                    if (c == 32) {
+                        c += __popc(__ballot_sync(0xffffffffu, a1 > -P.prune));
+                        if (c == 64) {
+                            c += __popc(__ballot_sync(0xffffffffu, a2 > -P.prune));
+                            c += __popc(__ballot_sync(0xffffffffu, a3 > -P.prune));
+                        }
+                    }
+                    if (lane == g + k) cnt = c;
+                }
+                __syncwarp();
+                // the butterfly adds lanes 16 apart, then 8, 4, 2, 1
+                const float2* p = wait + (lane >> 2) * kOrWait + (lane & 3);
+                float2 x[8];
+#pragma unroll
+                for (int k = 0; k < 8; k++) x[k] = p[4 * k];
+                float r0 = ((x[0].x + x[4].x) + (x[2].x + x[6].x)) + ((x[1].x + x[5].x) + (x[3].x + x[7].x));
+                float r1 = ((x[0].y + x[4].y) + (x[2].y + x[6].y)) + ((x[1].y + x[5].y) + (x[3].y + x[7].y));
+                r0 += __shfl_xor_sync(0xffffffffu, r0, 2); r1 += __shfl_xor_sync(0xffffffffu, r1, 2);
+                r0 += __shfl_xor_sync(0xffffffffu, r0, 1); r1 += __shfl_xor_sync(0xffffffffu, r1, 1);
+                const int from = ((lane - g) & 7) * 4;
+                r0 = __shfl_sync(0xffffffffu, r0, from); r1 = __shfl_sync(0xffffffffu, r1, from);
+                if ((lane & ~7) == g) { sum = r0; px = r1; }
+                __syncwarp();
+            }
+            // ---- lane = pair ----
+            float ref = 0.f, qk = 0.f;
+            if (on) {
+                if (__ldg(A.edges + A.E + e) != j) atomicOr(&g_status, CFB200_ST_PAIR_LAYOUT);       // not the dense layout
+                ref = __ldg(A.list + (size_t)e * kListStride);
+                const float* qp = A.qs + ih * kAtHd;
+                const float* kp = A.k + (j * H + h) * kAtHd;
+                float x[kAtHd];
+                if (vec) {
+#pragma unroll
+                    for (int d = 0; d < kAtHd / 4; d++) {
+                        const float4 u = __ldg(reinterpret_cast<const float4*>(qp) + d), v = __ldg(reinterpret_cast<const float4*>(kp) + d);
+                        x[4 * d] = __fmul_rn(u.x, v.x); x[4 * d + 1] = __fmul_rn(u.y, v.y);
+                        x[4 * d + 2] = __fmul_rn(u.z, v.z); x[4 * d + 3] = __fmul_rn(u.w, v.w);
+                    }
+                } else {
+#pragma unroll
+                    for (int d = 0; d < kAtHd; d++) x[d] = __fmul_rn(__ldg(qp + d), __ldg(kp + d));
+                }
+#pragma unroll
+                for (int o = 8; o > 0; o >>= 1)
+#pragma unroll
+                    for (int d = 0; d < o; d++) x[d] = __fadd_rn(x[d], x[d + o]);
+                qk = x[0];
+                cnt = max(cnt, 1);          // the nearest translation always counts (a coefficient that is not a number)
+            }
+            const float inv = 1.0f / sum;
+            const float zv = logf(sum) + ref * a;
+            const float sj = qk + zv;
+            float mx = on ? sj : -INFINITY;                 // running maximum up to this pair
+            if (lane == 0) mx = fmaxf(m, mx);
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) { const float u = __shfl_up_sync(0xffffffffu, mx, o); if (lane >= o) mx = fmaxf(u, mx); }
+            float before = __shfl_up_sync(0xffffffffu, mx, 1);
+            if (lane == 0) before = m;
+            const float sc = __expf(before - mx), p = __expf(sj - mx);
+            m = __shfl_sync(0xffffffffu, mx, 31);
+            if (on) {
+                A.z[e * H + h] = zv;
+                A.px[e * H + h] = px * inv;
+                pairs[lane] = make_float4(sc, p, p * inv, inv);
+            }
+            // ---- translations, as in attn_tile_kernel ----
+            int pre = cnt;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) { const int u = __shfl_up_sync(0xffffffffu, pre, o); if (lane >= o) pre += u; }
+            const int total = __shfl_sync(0xffffffffu, pre, 31);
+            pre -= cnt;
+            for (int f0 = 0; f0 < total; f0 += 32) {
+                const int idx = f0 + lane;
+                int jj = 0;                                 // the pair translation idx belongs to: the last with pre <= idx
+#pragma unroll
+                for (int o = 16; o > 0; o >>= 1) {
+                    const int u = __shfl_sync(0xffffffffu, pre, jj + o);
+                    if (u <= idx) jj += o;
+                }
+                jj = min(jj, nt - 1);
+                const int k = idx - __shfl_sync(0xffffffffu, pre, jj), cj = __shfl_sync(0xffffffffu, cnt, jj);
+                const float rj = __shfl_sync(0xffffffffu, ref, jj);
+                if (idx < total) {
+                    const float* Lp = A.list + (size_t)(e0 + tile0 + jj) * kListStride + k;
+                    const float d2 = __ldg(Lp);
+                    fw_record<2>(A, P, ih, rec + lane * kFwRec, a * (d2 - rj), d2, __ldg(Lp + kListLen), __ldg(Lp + 2 * kListLen),
+                                 __ldg(Lp + 3 * kListLen), d2, k == cj - 1 ? jj + 1 : 0);
+                }
+                __syncwarp();
+                const float4* R = reinterpret_cast<const float4*>(rec);
+                const int n = min(32, total - f0);
+                for (int r = 0; r < n; r++, R += kFwRec / 4) {
+                    const float4 u = R[0];
+                    const float d2 = u.z;
+                    const int flag = __float_as_int(u.w);
+                    fw_gaussians<2, true>(L, R, u, [&](const int x, const float g) { s[x] += g; T[x] = fmaf(g, d2, T[x]); });
+                    if (flag) flush(flag - 1);
+                }
+                __syncwarp();
+            }
+        }
+        const float inv_l = np > 0 ? 1.0f / l : 0.f;
+        const bool partial = TASKS && row >= (int)A.N;
+        const int64_t rh = (int64_t)(partial ? row - (int)A.N : row) * H + h;
+        if (lane == 0) (partial ? A.part_lse : A.lse)[rh] = m + logf(l);
+        float* sp = (partial ? A.part_spool : A.spool) + rh * kAtK + lane;
+#pragma unroll
+        for (int x = 0; x < 4; x++) {
+            float s0, s1, t0, t1;
+            unpack2(S[x], s0, s1); unpack2(Tq[x], t0, t1);
+            if (x == 0) {
+                sp[0] = s0 * inv_l; sp[32] = s1 * inv_l;
+                rows[lane] = t0 * inv_l * P.c_dist; rows[32 + lane] = t1 * inv_l * P.c_dist;
+            } else {
+                sp[64 * x] = s0 * inv_l * P.c_ang; sp[64 * x + 32] = s1 * inv_l * P.c_ang;
+                float* w = rows + 64 * x + (x > 1 ? kOrGap : 0) + lane;
+                w[0] = t0 * inv_l * P.c_ang; w[32] = t1 * inv_l * P.c_ang;
             }
         }
         __syncwarp();
-        const float up_d = project_row(W_s, srow, lane);     // W (pooled d^2-weighted sums)
+        const float up_d = project_row<kOrRow, kOrGap>(W_s, rows, lane);     // W (pooled d^2-weighted sums)
         if (lane < kAtHd) {
-            (partial ? A.part_out : A.out)[(row * H + h) * kAtHd + lane] = V * inv_l;
-            (partial ? A.part_upool : A.upool)[(row * H + h) * kAtHd + lane] = up_d;
+            (partial ? A.part_out : A.out)[rh * kAtHd + lane] = V * inv_l;
+            (partial ? A.part_upool : A.upool)[rh * kAtHd + lane] = up_d;
         }
         __syncwarp();
     }
@@ -1276,6 +1649,24 @@ static int launch_pairwise(const AtArgs& A, const Params& P, cudaStream_t st)
     return cudaGetLastError() == cudaSuccess ? CFB200_OK : CFB200_E_CUDA;
 }
 
+template <bool TASKS>
+static int launch_ordered(const AtArgs& A0, const Params& P, cudaStream_t st)
+{
+    AtArgs A = A0;
+    A.vec = on_grid({A.qs, A.k});
+    auto kern = attn_ordered_kernel<TASKS>;
+    static std::atomic<bool> attr_done[64];
+    int dev = 0;
+    cudaGetDevice(&dev);
+    if (!attr_done[dev & 63]) {
+        if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kOrSmem) != cudaSuccess) return CFB200_E_CUDA;
+        attr_done[dev & 63] = true;
+    }
+    kern<<<dim3(pairwise_grid_x(A.N, P.H), P.H), kOrWarps * 32, kOrSmem, st>>>(A, P);
+    if (TASKS) attn_merge_fwd_kernel<<<dim3(kSplitSlots / 8, P.H), 256, 0, st>>>(A, P.H);
+    return cudaGetLastError() == cudaSuccess ? CFB200_OK : CFB200_E_CUDA;
+}
+
 template <int MODE>
 static int launch_tile(const AtArgs& A0, const Params& P, cudaStream_t st)
 {
@@ -1299,6 +1690,7 @@ int attn_fused_fwd(const AtArgs& A, const Params& P, cudaStream_t st)
     // lists 5.5 against 6.3 ms).
     if (A.val != nullptr && (A.pairwise || A.list == nullptr)) {
         if (!A.counters_zeroed && cudaMemsetAsync(A.counters, 0, sizeof(int) * P.H, st) != cudaSuccess) return CFB200_E_CUDA;
+        if (A.list != nullptr && A.W[1] != nullptr) return A.tasks != nullptr ? launch_ordered<true>(A, P, st) : launch_ordered<false>(A, P, st);
         if (A.tasks != nullptr) return A.W[1] != nullptr ? launch_pairwise<true, true>(A, P, st) : launch_pairwise<false, true>(A, P, st);
         return A.W[1] != nullptr ? launch_pairwise<true, false>(A, P, st) : launch_pairwise<false, false>(A, P, st);
     }

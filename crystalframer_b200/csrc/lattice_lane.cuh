@@ -25,6 +25,7 @@ struct LatticeLane {
     static constexpr bool REFZ = MODE == 1;       // ref is the pair's z (else d^2_min, found here)
     // per-lane basis constants, pre-scaled so that a Gaussian is ex2(-b*b)
     float cd_lo, cd_hi, ca_lo, ca_hi;
+    float dstep, nastep;        // mode 2: the constants above are the indices' numbers, these the steps (negative for angles)
     float inv_d_interval, d_cut_scaled, xd_scale, inv_a_interval, xa_scale;
     unsigned win_d, win_a;
     bool wide_d;
@@ -40,13 +41,15 @@ struct LatticeLane {
     __device__ __forceinline__ void init(const Params& P, int lane_, float* records)
     {
         lane = lane_;
-        const float dstep = P.d_step * kLlSqrtLog2e, astep = P.a_step * kLlSqrtLog2e;
-        cd_lo = (float)(lane + 1) * dstep; cd_hi = (float)(lane + 33) * dstep;
+        const float dst = P.d_step * kLlSqrtLog2e, astep = P.a_step * kLlSqrtLog2e;
+        dstep = dst; nastep = -astep;
         // angle Gaussian k sits at (angle_dim - 1 - k) steps; this lane owns k = lane and k = lane + 32
-        ca_lo = (float)(P.angle_dim - 1 - lane) * astep; ca_hi = (float)(P.angle_dim - 33 - lane) * astep;
+        const float f = MODE == 2 ? 1.0f : dst, g = MODE == 2 ? 1.0f : astep;
+        cd_lo = (float)(lane + 1) * f; cd_hi = (float)(lane + 33) * f;
+        ca_lo = (float)(P.angle_dim - 1 - lane) * g; ca_hi = (float)(P.angle_dim - 33 - lane) * g;
         win_d = (unsigned)P.win_dist; win_a = (unsigned)P.win_ang;
         inv_d_interval = 1.0f / P.d_interval; d_cut_scaled = P.d_cut / P.d_interval;
-        xd_scale = dstep / P.d_interval;
+        xd_scale = dst / P.d_interval;
         inv_a_interval = P.angle_dim > 1 ? 1.0f / P.a_interval : 0.0f;
         xa_scale = P.a_sigma_inv * kLlSqrtLog2e;
         wide_d = P.win_dist > 32;
@@ -70,6 +73,11 @@ struct LatticeLane {
         if (BWD) px_l = fmaf(w, d2, px_l);
         return arg;
     }
+
+    // Arguments of the Gaussians: x + constant.  Mode 2, whose rounding is part of its result, adds number times step in one
+    // rounding, which the compiler may or may not do with a constant that is a product.
+    __device__ __forceinline__ float arg_d(const float x, const float c) const { return MODE == 2 ? fmaf(c, dstep, x) : x + c; }
+    __device__ __forceinline__ float arg_a(const float x, const float c) const { return MODE == 2 ? fmaf(c, nastep, x) : x - c; }
 
     // One group of up to 32 translations, one per lane: window records of the lanes that keep theirs, then
     // the walk over these survivors.  (dx, dy, dz) is read only where keep is set.
@@ -126,12 +134,12 @@ struct LatticeLane {
                 const int lo = (int)__byte_perm((unsigned)lo_pack, 0u, 0x4440);
                 const bool in0 = (unsigned)(lane - lo) < win_d, in1 = (unsigned)(lane + 32 - lo) < win_d;
                 if (!wide_d) {
-                    const float b = r0.y + (in1 ? cd_hi : cd_lo);
+                    const float b = arg_d(r0.y, in1 ? cd_hi : cd_lo);
                     const float g = ex2_approx(fmaf(-b, b, lw));
                     if (in0) { sd[0] += g; if (BWD) qd[0] = fmaf(g, d2s, qd[0]); }
                     if (in1) { sd[1] += g; if (BWD) qd[1] = fmaf(g, d2s, qd[1]); }
                 } else {
-                    const float b0 = r0.y + cd_lo, b1 = r0.y + cd_hi;
+                    const float b0 = arg_d(r0.y, cd_lo), b1 = arg_d(r0.y, cd_hi);
                     const float g0 = ex2_approx(fmaf(-b0, b0, lw)), g1 = ex2_approx(fmaf(-b1, b1, lw));
                     if (in0) { sd[0] += g0; if (BWD) qd[0] = fmaf(g0, d2s, qd[0]); }
                     if (in1) { sd[1] += g1; if (BWD) qd[1] = fmaf(g1, d2s, qd[1]); }
@@ -142,7 +150,7 @@ struct LatticeLane {
 #pragma unroll
                 for (int x = 0; x < 3; x++) {
                     const int lo = (int)__byte_perm((unsigned)lo_pack, 0u, 0x4441 + x);
-                    const float b0 = xa[x] - ca_lo, b1 = xa[x] - ca_hi;
+                    const float b0 = arg_a(xa[x], ca_lo), b1 = arg_a(xa[x], ca_hi);
                     const float g0 = ex2_approx(fmaf(-b0, b0, lw)), g1 = ex2_approx(fmaf(-b1, b1, lw));
                     if ((unsigned)(lane - lo) < win_a) { sa[x][0] += g0; if (BWD) qa[x][0] = fmaf(g0, d2s, qa[x][0]); }
                     if ((unsigned)(lane + 32 - lo) < win_a) { sa[x][1] += g1; if (BWD) qa[x][1] = fmaf(g1, d2s, qa[x][1]); }

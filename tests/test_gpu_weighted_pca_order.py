@@ -55,6 +55,28 @@ def test_training_forward_repeats_to_the_bit(row):
     assert outputs(BATCHES[row], cuda()) == want
 
 
+# small cells and Gaussians three times as wide: ranges beyond the lists beside ranges within; recorded before the sums of
+# tasks with lists were formed in tiles
+WIDE = [(6, 4, 40, 4.0, 12.0, 32, 6), (8, 1, 64, 3.0, 15.0, 16, 11), (12, 4, 40, 4.0, 12.0, 64, 18)]
+WIDE_GOLDEN = os.path.join(os.path.dirname(GOLDEN), "weighted_pca_wide_outputs.json")
+
+
+def wide_outputs(spec, dev):
+    model, tb = _model_and_batch(*spec, dev, layers=2)
+    with torch.no_grad():
+        for n, p in model.named_parameters():
+            if "lattice_pos" in n:
+                p.mul_(3.0)
+    return _predict(model, tb, spec[-1]).detach().cpu().numpy().ravel().view(np.uint32).tolist()
+
+
+@pytest.mark.parametrize("row", range(len(WIDE)))
+def test_training_forward_of_wide_gaussians_repeats_to_the_bit(row):
+    with open(WIDE_GOLDEN) as f:
+        want = json.load(f)[row]
+    assert wide_outputs(WIDE[row], cuda()) == want
+
+
 @pytest.mark.parametrize("sizes", [(1, 2, 3, 5, 31, 32, 33, 65)])
 @pytest.mark.parametrize("angles", [16, 64])
 @pytest.mark.parametrize("chunked", [False, True])
