@@ -1411,75 +1411,71 @@ __global__ void __launch_bounds__(kOrWarps * 32, 2) attn_ordered_kernel(const __
     }   // heads in turn
 }
 
-// Backward pass from the results of the training forward: warp = (atom, head), lane = pair (32 at a time).  Per pair
+// Backward pass from the results of the training forward.  Per pair
 //   p = exp(q.k + z - lse),  gz = p (gout . (v_j + values_ij) - gout . out_i),
 //   ga += c_dist x gz - p x gout . values_ij,  gq += gz k_j;   and ga += gout . upool once per atom
-// (the coefficient gradient as in the recomputing backward, reference quirk included).  The 16-component dot products run inside
-// the lanes; the 17 per-atom sums are reduced over the lanes once at the end, in a fixed order.
-__global__ void __launch_bounds__(256) attn_bwd_saved_kernel(const AtArgs A, const Params P)
+// (the coefficient gradient as in the recomputing backward, reference quirk included).  Block = (atom, eight heads), lane =
+// (head, four of the 16 components), so that a row of keys, values or value encodings is one contiguous 512-byte read: a lane
+// that took a whole head's 64 bytes would touch a cache line per lane and load, and the tags of the L1 cache set the pace (12
+// LDG.128 x 32 lines for 32 pairs of a head).  The dot products meet over four lanes.  Eight warps share the atom's pairs, one
+// pair at a time each: latency is covered by warps (64 registers, 32 warps per SM), which does better than two or four pairs in
+// flight per warp.  Bound by the latency of the reads.  Per launch, 256 log-normal crystals 49 -> 27 us (two pairs in flight 38),
+// 16 cells of 100-200 atoms 145 -> 72 us (111).
+constexpr int kBsWarps = 8;
+
+__device__ __forceinline__ float quad_sum(float v)
 {
-    const int lane = threadIdx.x & 31, H = P.H;
-    const int64_t task = (int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
-    if (task >= A.N * H) return;
-    const int64_t i = task / H;
-    const int h = (int)(task - i * H);
-    float q[kAtHd], g[kAtHd], gq[kAtHd];
-    float D = 0.f, gup = 0.f;
-    {
-        const float4* q4 = reinterpret_cast<const float4*>(A.qs + (i * H + h) * kAtHd);
-        const float4* g4 = reinterpret_cast<const float4*>(A.gout + (i * H + h) * kAtHd);
-        const float4* o4 = reinterpret_cast<const float4*>(A.out + (i * H + h) * kAtHd);
-        const float4* u4 = reinterpret_cast<const float4*>(A.upool + (i * H + h) * kAtHd);
-#pragma unroll
-        for (int c = 0; c < kAtHd / 4; c++) {
-            const float4 a = __ldg(q4 + c), b = __ldg(g4 + c), o = __ldg(o4 + c), u = __ldg(u4 + c);
-            q[4 * c] = a.x; q[4 * c + 1] = a.y; q[4 * c + 2] = a.z; q[4 * c + 3] = a.w;
-            g[4 * c] = b.x; g[4 * c + 1] = b.y; g[4 * c + 2] = b.z; g[4 * c + 3] = b.w;
-            D = fmaf(b.x, o.x, fmaf(b.y, o.y, fmaf(b.z, o.z, fmaf(b.w, o.w, D))));
-            gup = fmaf(b.x, u.x, fmaf(b.y, u.y, fmaf(b.z, u.z, fmaf(b.w, u.w, gup))));
-        }
-#pragma unroll
-        for (int c = 0; c < kAtHd; c++) gq[c] = 0.f;
-    }
-    const float lse = __ldg(A.lse + i * H + h);
+    v += __shfl_xor_sync(0xffffffffu, v, 1);
+    return v + __shfl_xor_sync(0xffffffffu, v, 2);
+}
+
+__device__ __forceinline__ float dot4(const float4 a, const float4 b) { return fmaf(a.x, b.x, fmaf(a.y, b.y, fmaf(a.z, b.z, a.w * b.w))); }
+
+__global__ void __launch_bounds__(kBsWarps * 32) attn_bwd_saved_kernel(const AtArgs A, const Params P)
+{
+    const int H = P.H, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int64_t i = blockIdx.x;
+    const int head = blockIdx.y * 8 + (lane >> 2), h = min(head, H - 1);       // lanes beyond the last head repeat it
+    const bool live = head < H;
+    const int64_t ih = i * H + h;
+    const int c0 = (lane & 3) * 4;
+    auto load4 = [&](const float* src, const int64_t row) { return __ldg(reinterpret_cast<const float4*>(src + row * kAtHd + c0)); };
+    const float4 q = load4(A.qs, ih), g = load4(A.gout, ih);
+    const float D = quad_sum(dot4(g, load4(A.out, ih)));
+    const float lse = __ldg(A.lse + ih);
     const int64_t e0 = A.e_start[i], e1 = A.e_start[i + 1];
     const int64_t j0 = e1 > e0 ? A.edges[A.E + e0] : 0;
+    float4 gq = make_float4(0.f, 0.f, 0.f, 0.f);
     float ga = 0.f;
-    for (int64_t e = e0 + lane; e < e1; e += 32) {
+#pragma unroll 1
+    for (int64_t e = e0 + warp; e < e1; e += kBsWarps) {
         const int64_t j = j0 + (e - e0);
-        const float4* k4 = reinterpret_cast<const float4*>(A.k + (j * H + h) * kAtHd);
-        const float4* v4 = reinterpret_cast<const float4*>(A.v + (j * H + h) * kAtHd);
-        const float4* x4 = reinterpret_cast<const float4*>(A.val + (e * H + h) * kAtHd);
-        const float zin = __ldg(A.z_in + e * H + h), px = __ldg(A.px + e * H + h);
-        float kk[kAtHd];
-        float qk = 0.f, gov = 0.f, cB = 0.f;
-#pragma unroll
-        for (int c = 0; c < kAtHd / 4; c++) {
-            const float4 a = __ldg(k4 + c), b = __ldg(v4 + c), x = __ldg(x4 + c);
-            kk[4 * c] = a.x; kk[4 * c + 1] = a.y; kk[4 * c + 2] = a.z; kk[4 * c + 3] = a.w;
-            qk = fmaf(q[4 * c], a.x, fmaf(q[4 * c + 1], a.y, fmaf(q[4 * c + 2], a.z, fmaf(q[4 * c + 3], a.w, qk))));
-            gov = fmaf(g[4 * c], b.x, fmaf(g[4 * c + 1], b.y, fmaf(g[4 * c + 2], b.z, fmaf(g[4 * c + 3], b.w, gov))));
-            cB = fmaf(g[4 * c], x.x, fmaf(g[4 * c + 1], x.y, fmaf(g[4 * c + 2], x.z, fmaf(g[4 * c + 3], x.w, cB))));
-        }
-        const float p_att = __expf(qk + zin - lse);
-        const float gzv = p_att * (gov + cB - D);
-        A.gz[e * H + h] = gzv;
-        ga += px * fmaf(P.c_dist, gzv, -p_att * cB);
-#pragma unroll
-        for (int c = 0; c < kAtHd; c++) gq[c] = fmaf(gzv, kk[c], gq[c]);
+        const float4 k = load4(A.k, j * H + h), v = load4(A.v, j * H + h), x = load4(A.val, e * H + h);
+        const float z = __ldg(A.z_in + e * H + h), px = __ldg(A.px + e * H + h);
+        const float qk = quad_sum(dot4(q, k)), gov = quad_sum(dot4(g, v)), cB = quad_sum(dot4(g, x));
+        const float p = __expf(qk + z - lse);
+        const float gz = p * (gov + cB - D);
+        if (live && (lane & 3) == 0) A.gz[e * H + h] = gz;
+        ga += px * fmaf(P.c_dist, gz, -p * cB);
+        gq.x = fmaf(gz, k.x, gq.x); gq.y = fmaf(gz, k.y, gq.y); gq.z = fmaf(gz, k.z, gq.z); gq.w = fmaf(gz, k.w, gq.w);
     }
-    // the lanes' sums, one butterfly per value (fixed order)
+    // the warps' parts, in a fixed order
+    __shared__ float part[kBsWarps][5][32];
+    part[warp][0][lane] = gq.x; part[warp][1][lane] = gq.y; part[warp][2][lane] = gq.z; part[warp][3][lane] = gq.w;
+    part[warp][4][lane] = ga;
+    __syncthreads();
+    if (warp > 0) return;
+    float r[5];
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-        ga += __shfl_xor_sync(0xffffffffu, ga, o);
-#pragma unroll
-        for (int c = 0; c < kAtHd; c++) gq[c] += __shfl_xor_sync(0xffffffffu, gq[c], o);
+    for (int c = 0; c < 5; c++) {
+        static_assert(kBsWarps == 8, "");
+        r[c] = ((part[0][c][lane] + part[1][c][lane]) + (part[2][c][lane] + part[3][c][lane])) +
+               ((part[4][c][lane] + part[5][c][lane]) + (part[6][c][lane] + part[7][c][lane]));
     }
-    if (lane == 0) A.ga[i * H + h] = ga + gup;
-    if (lane == 0) {
-        float4* o4 = reinterpret_cast<float4*>(A.gq + (i * H + h) * kAtHd);
-#pragma unroll
-        for (int c = 0; c < kAtHd / 4; c++) o4[c] = make_float4(gq[4 * c], gq[4 * c + 1], gq[4 * c + 2], gq[4 * c + 3]);
+    const float gup = quad_sum(dot4(g, load4(A.upool, ih)));
+    if (live) {
+        *reinterpret_cast<float4*>(A.gq + ih * kAtHd + c0) = make_float4(r[0], r[1], r[2], r[3]);
+        if ((lane & 3) == 0) A.ga[ih] = r[4] + gup;
     }
 }
 
@@ -1703,8 +1699,7 @@ int attn_fused_bwd(const AtArgs& A, const Params& P, cudaStream_t st)
     if (A.N == 0) return CFB200_OK;
     if (A.val == nullptr) return launch_tile<2>(A, P, st);
     if (!on_grid({A.qs, A.k, A.v, A.gout, A.out, A.upool, A.val, A.gq})) return CFB200_E_SHAPE;
-    const int64_t tasks = A.N * P.H;
-    attn_bwd_saved_kernel<<<(unsigned)((tasks + 7) / 8), 256, 0, st>>>(A, P);
+    attn_bwd_saved_kernel<<<dim3((unsigned)A.N, (unsigned)((P.H + 7) / 8)), kBsWarps * 32, 0, st>>>(A, P);
     return cudaGetLastError() == cudaSuccess ? CFB200_OK : CFB200_E_CUDA;
 }
 
