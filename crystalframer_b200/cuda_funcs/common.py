@@ -1,4 +1,5 @@
 """Helpers shared by the autograd Functions."""
+import time
 import weakref
 
 import torch
@@ -47,7 +48,8 @@ PAIR_LIST_BYTES_PER_PAIR = 5 * 128 * 4   # five planes of 128 floats: 2.5 KB of 
 PAIR_LIST_MAX_PAIRS = 4_000_000          # hard cap (10 GB); below it the list also has to fit a quarter of the free memory
 
 
-_FREE_MEMORY = {}          # device -> (free bytes at the last query, requests it may still serve)
+_FREE_MEMORY = {}          # device -> (free bytes at the last query, when that was)
+FREE_MEMORY_SECONDS = 10.0
 
 
 def pair_list_fits(num_pairs, device):
@@ -57,13 +59,27 @@ def pair_list_fits(num_pairs, device):
     if num_pairs > PAIR_LIST_MAX_PAIRS:
         return False
     need = num_pairs * PAIR_LIST_BYTES_PER_PAIR
-    # the driver query costs as much as several kernel launches: a recent answer serves requests far below it
+    # The driver query can take tens of milliseconds (41 ms measured; asked every 64 batches it was a third of a training
+    # step of 8 crystals): an answer of the last ten seconds serves requests far below it.
     key = (device.type, device.index)
-    free, uses = _FREE_MEMORY.get(key, (0, 0))
-    if uses <= 0 or need > free // 32:
-        free, uses = torch.cuda.mem_get_info(device)[0], 64
-    _FREE_MEMORY[key] = (free, uses - 1)
+    now = time.monotonic()
+    free, asked = _FREE_MEMORY.get(key, (0, 0.0))
+    if need > free // 32 or now - asked > FREE_MEMORY_SECONDS:
+        free = torch.cuda.mem_get_info(device)[0]
+        _FREE_MEMORY[key] = (free, now)
     return need <= free // 4
+
+
+def allocate_pair_list(num_pairs, device):
+    """Room for a batch's translation lists, or None where they do not fit (also where the memory went since it was asked
+    for)."""
+    if not pair_list_fits(num_pairs, device):
+        return None
+    try:
+        return torch.empty((num_pairs, 5, 128), dtype=torch.float32, device=device)
+    except torch.OutOfMemoryError:
+        _FREE_MEMORY.pop((device.type, device.index), None)
+        return None
 
 
 def pair_geometry(rpos_ij_e, tvecs_n, batch_i, edge_ij_e, cutoff):
@@ -91,8 +107,8 @@ def pair_geometry(rpos_ij_e, tvecs_n, batch_i, edge_ij_e, cutoff):
     N, E = batch.shape[0], edges.shape[1]
     cache = torch.empty((E, 4), device=dev, dtype=torch.float32)
     plist = None
-    if (2 * rng + 1) ** 3 <= 128 and pair_list_fits(E, dev):
-        plist = torch.empty((E, 5, 128), device=dev, dtype=torch.float32)
+    if (2 * rng + 1) ** 3 <= 128:
+        plist = allocate_pair_list(E, dev)
     _lib.invoke("cfb200_pair_cache", 2, dev, _lib.ptr(pos), _lib.ptr(tv), _lib.iptr(batch), _lib.iptr(edges), N, E, rng,
                 _lib.ptr(cache), _lib.ptr(plist))
     for k in [k for k, v in _pair_cache.items() if v[0]() is None]:      # lists are large: drop dead batches at once

@@ -80,14 +80,14 @@ class LayerGeometry:
     def from_raw(cls, pos, trans, sizes, N, E, cutoff, pairwise=False):
         """One call of cfb200_batch_geometry on raw positions (N,3), lattice vectors (B,3,3), sizes (B).  ``pairwise``: the
         work queue is cut for the training forward of weighted-PCA models (attn_pairwise_kernel)."""
-        from .cuda_funcs.common import pair_list_fits
+        from .cuda_funcs.common import allocate_pair_list
         from .cuda_funcs.kernel_manager import KernelManager
         g = cls()
         dev = pos.device
         B = trans.shape[0]
         cfg = KernelManager.config
         rng = int(cfg.lattice_range if cutoff == 0.0 else cfg.minimum_range)
-        want_list = rng > 0 and (2 * rng + 1) ** 3 <= 128 and pair_list_fits(E, dev)
+        want_list = rng > 0 and (2 * rng + 1) ** 3 <= 128
         # int64 block: edges (2E) | e_start (N+1) | batch (N) | crystal_start (B+1)
         o_es = 2 * E
         o_b = o_es + N + 1
@@ -104,7 +104,7 @@ class LayerGeometry:
         o_sp = _align(o_ct + 64)
         o_ws = _align(o_sp + n_split)
         fbuf = torch.empty(o_ws + ws_bytes // 4, dtype=torch.float32, device=dev)
-        plist = torch.empty((E, 5, 128), dtype=torch.float32, device=dev) if want_list else None
+        plist = allocate_pair_list(E, dev) if want_list else None
         ip, fp = ibuf.data_ptr(), fbuf.data_ptr()
         _lib.invoke("cfb200_batch_geometry_pairwise" if pairwise else "cfb200_batch_geometry", 7, dev, _lib.ptr(pos), _lib.ptr(trans), _lib.iptr(sizes), B, N, E, rng,
                     ip, ip + 8 * o_es, ip + 8 * o_b, ip + 8 * o_cs, fp, None, fp + 4 * o_rv, None,
@@ -136,7 +136,9 @@ class LayerGeometry:
         from .cuda_funcs.common import csr_offsets, pair_geometry
         g = cls()
         g.N, g.E, g.B = batch.shape[0], edges.shape[1], tvecs.shape[0]
-        g.pos_ij, g.tvecs, g.batch, g.edges, g.rvlen = pos_ij, tvecs, batch, edges, rvlen
+        # (the pair list's data, not the tensor: callers hang the geometry on that, and a cycle would keep a batch's lists, a
+        # hundred megabytes and more, until the garbage collector comes by)
+        g.pos_ij, g.tvecs, g.batch, g.edges, g.rvlen = pos_ij, tvecs, batch, edges.detach(), rvlen
         g.e_start = csr_offsets(edges, g.N)
         pair_cache, pair_list, g.cache_range = pair_geometry(pos_ij, tvecs, batch, edges, cutoff)
         pairs_per_atom = (g.e_start[1:] - g.e_start[:-1]).float()

@@ -453,3 +453,31 @@ def test_flat_adamw_matches_torch():
     # parameters stay views of the flat buffer, so state_dict round trips keep working
     ours.load_state_dict({k: v.clone() for k, v in ref.state_dict().items()})
     assert all(p.data_ptr() >= opt.flat.data_ptr() and p.data_ptr() < opt.flat.data_ptr() + 4 * opt.n for p in ours.parameters())
+
+
+def test_layers_called_with_tensors_leave_no_memory_behind():
+    """Layers that are handed a pair list keep a batch's geometry on it: it goes with the batch, without the garbage
+    collector (real- and reciprocal-space layers in turn take that way)."""
+    import gc
+    from crystalframer_b200 import data, synth
+    from crystalframer_b200.latticeformer import Latticeformer, ModelParams
+    dev = torch.device("cuda:0")
+    if not torch.cuda.is_available():
+        pytest.skip("no CUDA device")
+    torch.manual_seed(0)
+    model = Latticeformer(ModelParams(num_layers=2, frame_method="no", value_pe_angle_real=0, domain="real-reci")).to(dev).train()
+    tb = data.host_batch(synth.make_batch(16, 5), np.zeros((16, 1), np.float32), pinned=False).to(dev, non_blocking=False)
+
+    def step():
+        model.zero_grad(set_to_none=True)
+        model(tb).square().sum().backward()
+        return torch.cuda.memory_allocated()
+    step(), step()
+    gc.collect()
+    gc.disable()
+    try:
+        first = step()
+        last = [step() for _ in range(8)][-1]
+    finally:
+        gc.enable()
+    assert last - first < 1 << 20, (first, last)            # a batch's lists alone: some 5 MB

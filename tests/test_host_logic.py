@@ -229,3 +229,31 @@ def test_reference_checkpoint_layout_round_trip():
         assert torch.equal(v, src.state_dict()[k]), k
     with pytest.raises(KeyError):
         checkpoint.load_reference_checkpoint(live, ck, prefix="ema.")
+
+
+def test_free_memory_is_asked_for_rarely(monkeypatch):
+    """Translation lists: one driver query serves requests below a 32nd of what was free for ten seconds; larger requests and
+    later ones ask again; a quarter of what is free is the limit, and an allocation that fails means no lists."""
+    import torch
+    from crystalframer_b200.cuda_funcs import common
+    now, free, asked = [100.0], [64 * 2560 * 100], []
+    monkeypatch.setattr(common, "_FREE_MEMORY", {})
+    monkeypatch.setattr(common.time, "monotonic", lambda: now[0])
+    monkeypatch.setattr(torch.cuda, "mem_get_info", lambda d: (asked.append(d), (free[0], 1 << 40))[1])
+    dev = torch.device("cuda:0")
+    assert all(common.pair_list_fits(n, dev) for n in (1, 100, 200)) and len(asked) == 1
+    assert common.pair_list_fits(201, dev) and len(asked) == 2              # above a 32nd
+    assert common.pair_list_fits(1600, dev) and not common.pair_list_fits(1601, dev) and len(asked) == 4
+    now[0] += 9.0
+    assert common.pair_list_fits(5, dev) and len(asked) == 4
+    now[0] += 1.5
+    free[0] = 2560 * 8
+    assert not common.pair_list_fits(5, dev) and len(asked) == 5
+    assert not common.pair_list_fits(common.PAIR_LIST_MAX_PAIRS + 1, dev) and len(asked) == 5
+    assert common.allocate_pair_list(5, dev) is None
+
+    def full(*a, **k):
+        raise torch.OutOfMemoryError("full")
+    free[0] = 1 << 40
+    monkeypatch.setattr(torch, "empty", full)
+    assert common.allocate_pair_list(5, dev) is None and common._FREE_MEMORY == {}
