@@ -889,108 +889,133 @@ __global__ void __launch_bounds__(256) pair_cache_kernel(const float* __restrict
 // exp(a (d^2 - d^2_min)) falls with the distance, the translations a lattice-sum task has to expand, and the
 // candidates a second-axis search has to score, are a prefix of this list, whatever the head or the layer.
 
-// warp = one pair; lane l holds list positions l, l+32, l+64, l+96.  Keys are (bits of d^2) << 32 | index:
-// d^2 >= 0, so the unsigned order of the bits is the order of the values, and equal distances fall in
-// index order.  A bitonic network sorts the 128 keys: strides below 32 exchange between lanes, strides 32
-// and 64 between a lane's own registers.
-// It is bound by the network's instructions, so it first runs on 32-bit keys, the index in place of the distance's seven
-// last bits (half the exchanges, minimum and maximum in one instruction each); only where two neighbours then stand in the
-// wrong order -- distances within 2^-17 of one another, about one pair in twenty -- the exact keys are sorted.
+// warp = one pair at a time; lane l holds list positions 4 l .. 4 l + 3.  Keys are (bits of d^2) << 32 | index: d^2 >= 0, so
+// the unsigned order of the bits is the order of the values, and equal distances fall in index order.  A bitonic network sorts
+// the 128 keys, in the form whose merges begin with mirrored partners, so that the lower position always takes the smaller key:
+// 13 of its 28 steps are between a lane's own registers, minimum and maximum without a choice of direction, and 15 are
+// shuffles.  (With position = 32 r + lane and alternating directions 25 were shuffles.)  It first runs on 32-bit keys, the
+// index in place of the distance's seven last bits (half the exchanges); only where two neighbours then stand in the wrong
+// order -- distances within 2^-17 of one another, about one pair in twenty -- the exact keys are sorted.  Translations come
+// from a table in shared memory, four list positions leave in one 128-bit store per plane.
+// Bound by the network's instructions and, behind them, the 2.5 KB written per pair: 1.56 M pairs 1.65 -> 0.91 ms (0.61
+// for the writes alone), 42 k pairs 66 -> 41 us.
+constexpr int kPlWarps = 4, kPlPairs = 8;               // pairs that a warp sorts one after the other
+
+template <typename K>
+__device__ __forceinline__ void exchange(K& a, K& b)
+{
+    const K lo = min(a, b), hi = max(a, b);
+    a = lo; b = hi;
+}
+
 template <typename K>
 __device__ __forceinline__ void sort_list(K (&key)[4], const int lane)
 {
 #pragma unroll
     for (int k = 2; k <= kListLen; k <<= 1) {
+        // position i meets i ^ (k - 1), the mirror image in its group of k ...
+        if (k == 2) { exchange(key[0], key[1]); exchange(key[2], key[3]); }
+        else if (k == 4) { exchange(key[0], key[3]); exchange(key[1], key[2]); }
+        else {
+            const bool low = (lane & (k >> 3)) == 0;
+            K other[4];
 #pragma unroll
-        for (int j = k >> 1; j > 0; j >>= 1) {
-            if (j >= 32) {
-                const int dr = j >> 5;
+            for (int r = 0; r < 4; r++) other[r] = __shfl_xor_sync(0xffffffffu, key[3 - r], (k >> 2) - 1);
+#pragma unroll
+            for (int r = 0; r < 4; r++) key[r] = low ? min(key[r], other[r]) : max(key[r], other[r]);
+        }
+        // ... then i ^ j
+#pragma unroll
+        for (int j = k >> 2; j > 0; j >>= 1) {
+            if (j == 1) { exchange(key[0], key[1]); exchange(key[2], key[3]); }
+            else if (j == 2) { exchange(key[0], key[2]); exchange(key[1], key[3]); }
+            else {
+                const bool low = (lane & (j >> 2)) == 0;
 #pragma unroll
                 for (int r = 0; r < 4; r++) {
-                    if ((r & dr) == 0) {
-                        const bool up = (((r * 32 + lane) & k) == 0);
-                        const K lo = min(key[r], key[r | dr]), hi = max(key[r], key[r | dr]);
-                        key[r] = up ? lo : hi;
-                        key[r | dr] = up ? hi : lo;
-                    }
-                }
-            } else {
-#pragma unroll
-                for (int r = 0; r < 4; r++) {
-                    const K other = __shfl_xor_sync(0xffffffffu, key[r], j);
-                    const bool up = (((r * 32 + lane) & k) == 0);
-                    key[r] = ((lane & j) == 0) == up ? min(key[r], other) : max(key[r], other);
+                    const K other = __shfl_xor_sync(0xffffffffu, key[r], j >> 2);
+                    key[r] = low ? min(key[r], other) : max(key[r], other);
                 }
             }
         }
     }
 }
 
-__global__ void __launch_bounds__(128) pair_list_kernel(const float* __restrict__ pos_ij, const float* __restrict__ tvecs,
-                                                        const int64_t* __restrict__ batch, const int64_t* __restrict__ edges,
-                                                        int64_t E, int R, float* __restrict__ out)
+__global__ void __launch_bounds__(kPlWarps * 32) pair_list_kernel(const float* __restrict__ pos_ij, const float* __restrict__ tvecs,
+                                                                  const int64_t* __restrict__ batch, const int64_t* __restrict__ edges,
+                                                                  int64_t E, int R, int vec, float* __restrict__ out)
 {
+    __shared__ float4 table[kListLen];                  // n1, n2, n3 and code of a translation
     const int lane = threadIdx.x & 31;
-    const int64_t e = (int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
-    if (e >= E) return;
     const int L = 2 * R + 1, nT = L * L * L;
-    const int64_t c = batch[edges[e]];
-    const float* Tc = tvecs + 9 * c;
-    const float t1x = __ldg(Tc), t1y = __ldg(Tc + 1), t1z = __ldg(Tc + 2);
-    const float t2x = __ldg(Tc + 3), t2y = __ldg(Tc + 4), t2z = __ldg(Tc + 5);
-    const float t3x = __ldg(Tc + 6), t3y = __ldg(Tc + 7), t3z = __ldg(Tc + 8);
-    const float rx = __ldg(pos_ij + 3 * e), ry = __ldg(pos_ij + 3 * e + 1), rz = __ldg(pos_ij + 3 * e + 2);
-    auto separation_fused = [&](const int t, float& dx, float& dy, float& dz, float& d2, int& code) {
-        const int q = t / L, k1 = q / L, k2 = q - k1 * L, k3 = t - q * L;
-        const float n1 = (float)(k1 - R), n2 = (float)(k2 - R), n3 = (float)(k3 - R);
-        const float ox = fmaf(t3x, n3, fmaf(t2x, n2, rx)), oy = fmaf(t3y, n3, fmaf(t2y, n2, ry)), oz = fmaf(t3z, n3, fmaf(t2z, n2, rz));
-        dx = fmaf(t1x, n1, ox); dy = fmaf(t1y, n1, oy); dz = fmaf(t1z, n1, oz);
-        d2 = fmaf(dz, dz, fmaf(dy, dy, dx * dx));
-        code = k1 | (k2 << 8) | (k3 << 16) | (t << 24);
-    };
-    // the entries of the lane's list positions, translation t[r] at position r * 32 + lane
-    int t[4], code[4];
-    float dx[4], dy[4], dz[4], d2[4];
-    auto fill = [&]() {
-#pragma unroll
-        for (int r = 0; r < 4; r++) {
-            dx[r] = dy[r] = dz[r] = 0.f; d2[r] = 1e30f; code[r] = -1;
-            if (t[r] < nT) separation_fused(t[r], dx[r], dy[r], dz[r], d2[r], code[r]);
-        }
-    };
-#pragma unroll
-    for (int r = 0; r < 4; r++) t[r] = r * 32 + lane;
-    fill();
     {
-        unsigned key[4];
-#pragma unroll
-        for (int r = 0; r < 4; r++) key[r] = (__float_as_uint(d2[r]) & ~127u) | (unsigned)t[r];
-        sort_list(key, lane);
-#pragma unroll
-        for (int r = 0; r < 4; r++) t[r] = (int)(key[r] & 127u);
+        const int t = threadIdx.x;
+        static_assert(kPlWarps * 32 == kListLen, "");
+        const int q = t / L, k1 = q / L, k2 = q - k1 * L, k3 = t - q * L;
+        table[t] = make_float4((float)(k1 - R), (float)(k2 - R), (float)(k3 - R),
+                               __int_as_float(t < nT ? k1 | (k2 << 8) | (k3 << 16) | (t << 24) : -1));
     }
-    fill();
-    bool wrong = false;
+    __syncthreads();
+    const int64_t first = ((int64_t)blockIdx.x * kPlWarps + (threadIdx.x >> 5)) * kPlPairs;
+    for (int64_t e = first; e < min(first + kPlPairs, E); e++) {
+        const int64_t c = batch[edges[e]];
+        const float* Tc = tvecs + 9 * c;
+        const float t1x = __ldg(Tc), t1y = __ldg(Tc + 1), t1z = __ldg(Tc + 2);
+        const float t2x = __ldg(Tc + 3), t2y = __ldg(Tc + 4), t2z = __ldg(Tc + 5);
+        const float t3x = __ldg(Tc + 6), t3y = __ldg(Tc + 7), t3z = __ldg(Tc + 8);
+        const float rx = __ldg(pos_ij + 3 * e), ry = __ldg(pos_ij + 3 * e + 1), rz = __ldg(pos_ij + 3 * e + 2);
+        // the entries of the lane's list positions, translation t[r] at position 4 lane + r
+        int t[4];
+        float dx[4], dy[4], dz[4], d2[4], code[4];
+        auto fill = [&]() {
 #pragma unroll
-    for (int r = 0; r < 4; r++) {                       // the entry behind this one: the next lane's, or lane 0's of the next 32
-        const float behind = __shfl_sync(0xffffffffu, lane == 0 && r < 3 ? d2[r < 3 ? r + 1 : r] : d2[r], (lane + 1) & 31);
-        const float next = lane == 31 && r == 3 ? d2[r] : behind;
-        wrong |= !(d2[r] <= next);
-    }
-    if (__any_sync(0xffffffffu, wrong)) {
-        unsigned long long key[4];
+            for (int r = 0; r < 4; r++) {
+                const float4 n = table[t[r]];
+                const float ox = fmaf(t3x, n.z, fmaf(t2x, n.y, rx)), oy = fmaf(t3y, n.z, fmaf(t2y, n.y, ry)), oz = fmaf(t3z, n.z, fmaf(t2z, n.y, rz));
+                dx[r] = fmaf(t1x, n.x, ox); dy[r] = fmaf(t1y, n.x, oy); dz[r] = fmaf(t1z, n.x, oz);
+                d2[r] = fmaf(dz[r], dz[r], fmaf(dy[r], dy[r], dx[r] * dx[r]));
+                code[r] = n.w;
+                if (t[r] >= nT) { dx[r] = dy[r] = dz[r] = 0.f; d2[r] = 1e30f; }
+            }
+        };
 #pragma unroll
-        for (int r = 0; r < 4; r++) key[r] = ((unsigned long long)__float_as_uint(d2[r]) << 32) | (unsigned)t[r];
-        sort_list(key, lane);
-#pragma unroll
-        for (int r = 0; r < 4; r++) t[r] = (int)(unsigned)(key[r] & 0xffffffffull);
+        for (int r = 0; r < 4; r++) t[r] = r * 32 + lane;       // (any order; neighbouring lanes read neighbouring entries)
         fill();
-    }
-    float* o = out + (size_t)e * kListStride + lane;
+        {
+            unsigned key[4];
 #pragma unroll
-    for (int r = 0; r < 4; r++) {
-        o[r * 32] = d2[r]; o[kListLen + r * 32] = dx[r]; o[2 * kListLen + r * 32] = dy[r]; o[3 * kListLen + r * 32] = dz[r];
-        o[4 * kListLen + r * 32] = __int_as_float(code[r]);
+            for (int r = 0; r < 4; r++) key[r] = (__float_as_uint(d2[r]) & ~127u) | (unsigned)t[r];
+            sort_list(key, lane);
+#pragma unroll
+            for (int r = 0; r < 4; r++) t[r] = (int)(key[r] & 127u);
+        }
+        fill();
+        const float behind = __shfl_down_sync(0xffffffffu, d2[0], 1);
+        const bool wrong = !(d2[0] <= d2[1] && d2[1] <= d2[2] && d2[2] <= d2[3] && (lane == 31 || d2[3] <= behind));
+        if (__any_sync(0xffffffffu, wrong)) {
+            unsigned long long key[4];
+#pragma unroll
+            for (int r = 0; r < 4; r++) key[r] = ((unsigned long long)__float_as_uint(d2[r]) << 32) | (unsigned)t[r];
+            sort_list(key, lane);
+#pragma unroll
+            for (int r = 0; r < 4; r++) t[r] = (int)(unsigned)(key[r] & 0xffffffffull);
+            fill();
+        }
+        float* o = out + (size_t)e * kListStride + 4 * lane;
+        if (vec) {                                      // the lists are on the 16-byte grid
+            float4* o4 = reinterpret_cast<float4*>(o);
+            o4[0] = make_float4(d2[0], d2[1], d2[2], d2[3]);
+            o4[kListLen / 4] = make_float4(dx[0], dx[1], dx[2], dx[3]);
+            o4[2 * kListLen / 4] = make_float4(dy[0], dy[1], dy[2], dy[3]);
+            o4[3 * kListLen / 4] = make_float4(dz[0], dz[1], dz[2], dz[3]);
+            o4[4 * kListLen / 4] = make_float4(code[0], code[1], code[2], code[3]);
+        } else {
+#pragma unroll
+            for (int r = 0; r < 4; r++) {
+                o[r] = d2[r]; o[kListLen + r] = dx[r]; o[2 * kListLen + r] = dy[r]; o[3 * kListLen + r] = dz[r];
+                o[4 * kListLen + r] = code[r];
+            }
+        }
     }
 }
 
@@ -1003,7 +1028,8 @@ int pair_cache(const float* pos_ij, const float* tvecs, const int64_t* batch, co
                                                                       reinterpret_cast<float4*>(out));
     if (list != nullptr) {
         if ((2 * R + 1) * (2 * R + 1) * (2 * R + 1) > kListLen) return CFB200_E_UNSUPPORTED;
-        pair_list_kernel<<<(unsigned)((E + 3) / 4), 128, 0, st>>>(pos_ij, tvecs, batch, edges, E, R, list);
+        pair_list_kernel<<<(unsigned)((E + kPlWarps * kPlPairs - 1) / (kPlWarps * kPlPairs)), kPlWarps * 32, 0, st>>>(pos_ij, tvecs, batch, edges, E, R,
+                                                                                                        on_grid({list}), list);
     }
     return cudaGetLastError() == cudaSuccess ? CFB200_OK : CFB200_E_CUDA;
 }

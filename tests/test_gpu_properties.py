@@ -481,3 +481,46 @@ def test_layers_called_with_tensors_leave_no_memory_behind():
     finally:
         gc.enable()
     assert last - first < 1 << 20, (first, last)            # a batch's lists alone: some 5 MB
+
+
+@pytest.mark.parametrize("sizes", [(1,), (5, 2, 1, 1, 1), (1, 4, 4), (7, 9, 3)])        # 1, 32, 33 and 139 pairs
+@pytest.mark.parametrize("rng", [1, 2])
+@pytest.mark.parametrize("offset", [0, 1])
+def test_translation_lists_are_sorted(sizes, rng, offset):
+    """Every pair's list holds each translation of the box once, by distance and, where distances are equal (cubic cells with
+    atoms on a grid have many), by number; entries agree with float64 to rounding; padding is far away.  On the 16-byte grid
+    and off it."""
+    if not torch.cuda.is_available():
+        pytest.skip("no CUDA device")
+    from crystalframer_b200 import _lib, synth
+    from crystalframer_b200.encoder import build_pair_list
+    dev = torch.device("cuda:0")
+    b = synth.concat([synth.make_batch(1, 3 + n, size_dist="uniform", size_lo=n, size_hi=n, len_lo=3.0, len_hi=8.0) for n in sizes])
+    first = b.sizes[0]
+    b.trans_vec[0] = np.eye(3) * 4.0
+    b.pos[:first] = np.round(b.pos[:first])
+    t = lambda x, d: torch.from_numpy(np.ascontiguousarray(x, dtype=d)).to(dev)
+    edges, e_start, batch, _ = build_pair_list(t(b.sizes, np.int64))
+    pos, cells = t(b.pos, np.float32), t(b.trans_vec, np.float32)
+    pos_ij = (pos[edges[1]] - pos[edges[0]]).contiguous()
+    E, n = edges.shape[1], 2 * rng + 1
+    buf = torch.full((E * 640 + 8,), float("nan"), device=dev)
+    lists = buf[offset:offset + E * 640]
+    cache = torch.empty(E, 4, device=dev)
+    p = _lib.ptr
+    _lib.invoke("cfb200_pair_cache", 2, dev, p(pos_ij), p(cells), _lib.iptr(batch), _lib.iptr(edges), len(pos), E, rng, p(cache), p(lists))
+    assert buf[:offset].isnan().all() and buf[offset + E * 640:].isnan().all()
+    got = lists.view(E, 5, 128).cpu()
+    code = got[:, 4].contiguous().view(torch.int32)
+    nT = n ** 3
+    assert (code[:, nT:] == -1).all() and (got[:, 0, nT:] == 1e30).all() and (got[:, 1:4, nT:] == 0).all()
+    index = (code[:, :nT] >> 24) & 255
+    assert torch.equal(index.sort(1)[0], torch.arange(nT, dtype=torch.int32).expand(E, nT))
+    d2 = got[:, 0, :nT]
+    ahead, behind = d2[:, :-1], d2[:, 1:]
+    assert ((ahead < behind) | ((ahead == behind) & (index[:, :-1] < index[:, 1:]))).all()
+    cells_n = torch.stack([(code >> s) & 255 for s in (0, 8, 16)], -1)[:, :nT].double() - rng
+    want = pos_ij.double().cpu()[:, None] + torch.einsum("etk,ekd->etd", cells_n, cells.double().cpu()[batch.cpu()[edges[0].cpu()]])
+    xyz = got[:, 1:4, :nT].permute(0, 2, 1).double()
+    assert ((xyz - want).abs() <= 4 * 2.0 ** -24 * 40.0).all()              # three fused steps on numbers below 40
+    assert ((d2.double() - xyz.square().sum(-1)).abs() <= 3 * 2.0 ** -24 * xyz.square().sum(-1)).all()
