@@ -507,21 +507,27 @@ __device__ __forceinline__ float warp_max(float v)
 // share its lists in L1.
 //   First axis: lane = pair, tiles of 32: q.k, the pair's nearest image (cached geometry) and its score; arg-max over the
 //   lanes.
-//   Second axis: a pair's score is at most q.k + a d^2_min.  The pair with the highest such bound is searched first, the
-//   others only where their bound still reaches the best score so far.  A search runs with lane = translation: 32 entries
+//   Second axis: a pair's score is at most q.k + a d^2_min.  Lane = pair again, the pairs' nearest images give a score that
+//   is reached; the pair that reaches it is searched first, the others only where their bound still reaches the best score so
+//   far.  A search runs with lane = translation: 32 entries
 //   of the pair's sorted list at a time, until what follows cannot reach the best candidate.  Which pair and image win
 //   depends neither on the order nor on what is left out: what is left out could neither win nor tie.
-// Bound by the latency of its loads; no block barriers.  Per launch, against one thread per pair (max_frame_kernel): 64
-// crystals of 100-200 atoms 1.07 against 1.97 ms, 16 of them 0.30 / 0.52 ms; but 256 log-normal crystals (14 pairs per
-// atom, most of which have to be searched) 0.107 / 0.070 ms -- so max_frame() picks by pairs per atom.  A prediction of some
-// 4 000 atoms (four launches) with this kernel / the other: 20 pairs per atom 2.66 / 2.32 ms, 33 3.41 / 3.00, 45 3.56 / 3.27,
-// 66 4.15 / 4.21, 100 4.82 / 5.36, 159 5.86 / 7.41; 256 log-normal crystals with two of 200 atoms (42) 2.63 / 2.57, with six
-// (77) 4.10 / 4.35.
+// Bound by the latency of its loads; no block barriers.  Per launch 64 crystals of 100-200 atoms 0.64 ms, 16 of them 0.16
+// (without the nearest images 0.82 / 0.20: the pair with the highest bound is often a poor one, and four pairs are searched
+// for one; with q.k formed again for the second axis 1.00 / 0.24).  Against one thread per pair (max_frame_kernel), both sides
+// in us: 2 273 atoms of 14 pairs 86 / 71, 2 630 of 22 100 / 77, 3 072 of 32 125 / 121, 3 246 of 42 141 / 162, 3 831 of 72 199 /
+// 348, 2 534 of 165 202 / 516; one cell of 60 atoms, too few warps to cover the latency, 18 / 12 -- so max_frame() picks by
+// pairs per atom, and asks for more of them where atoms are few.
 constexpr int kFrWarps = 8;                // (atom, head) tasks per block
-constexpr int kFrWarpPairs = 64;           // pairs per atom above which this kernel runs
+constexpr int kFrWarpPairs = 36, kFrWarpPairsFew = 64;     // pairs per atom above which this kernel runs; with fewer than
+constexpr int64_t kFrManyTasks = 8192;                     // that many (atom, head) tasks
+// Pairs of an atom whose q.k and smallest d^2 are kept between the axes (a multiple of 32; those beyond are computed again): a
+// lane's key is 64 bytes of a line of its own.
+constexpr int kFrKept = 256;
 
 __global__ void __launch_bounds__(kFrWarps * 32, 3) max_frame_warp_kernel(const FrArgs A, const Params P)
 {
+    __shared__ float2 kept[kFrWarps][kFrKept];
     const int H = P.H, lane = threadIdx.x & 31;
     const int64_t task = (int64_t)blockIdx.x * kFrWarps + (threadIdx.x >> 5);
     if (task >= A.N * H) return;
@@ -555,6 +561,11 @@ __global__ void __launch_bounds__(kFrWarps * 32, 3) max_frame_warp_kernel(const 
     auto order_of = [](const unsigned long long key) { return (unsigned)(key >> 32); };
     const unsigned long long none = make_key(-1e10f, 0u);      // a score must exceed -1e10 to be selected
 
+    auto bound_of = [&](const float d, const float d2raw) {
+        if (!(a < 0.f) || A.is_static) return 3e38f;
+        const float g = a * d2raw;
+        return d + g + 1e-6f * (fabsf(d) + fabsf(g));                        // above any rounding of the score's sum
+    };
     // lane = pair: q.k, the first axis' candidate, and the bound on the second axis' score
     float dot = 0.f, known = -1.f, bound = -3e38f;
     auto first_pass = [&](const int t, const float amp1) {
@@ -579,14 +590,24 @@ __global__ void __launch_bounds__(kFrWarps * 32, 3) max_frame_warp_kernel(const 
             const bool hit = A.cache != nullptr && (same_box || (wider && __ldg(&A.cache[e].y) < reach2));
             cd = first_axis_candidate(cell, a, R1, R2, R3, amp1, A.seed1, (uint64_t)(e * H + h), hit ? A.cache + e : nullptr, C,
                                       hit && A.list != nullptr ? A.list + (size_t)e * kListStride : nullptr, reach2);
-            bound = 3e38f;
-            if (a < 0.f && !A.is_static) {
-                const float g = a * cd.d2raw;
-                bound = dot + g + 1e-6f * (fabsf(dot) + fabsf(g));           // above any rounding of the score's sum
-            }
+            bound = bound_of(dot, cd.d2raw);
         }
         known = cd.d2raw;
         return cd;
+    };
+    // the same lane's result of an earlier first_pass over the tile
+    auto restore = [&](const int t) {
+        dot = 0.f; bound = -3e38f; known = -1.f;
+        if (t < np) {
+            const float2 v = kept[threadIdx.x >> 5][t];
+            dot = v.x; known = v.y;
+            bound = bound_of(dot, known);
+        }
+    };
+
+    auto recall = [&](const int t0, const int t) {              // (one tile: still in registers)
+        if (t0 < kFrKept) restore(t);
+        else first_pass(t, 0.0f);
     };
 
     unsigned long long best1 = none, lead = 0ull;
@@ -595,6 +616,7 @@ __global__ void __launch_bounds__(kFrWarps * 32, 3) max_frame_warp_kernel(const 
         const int t = t0 + lane;
         const Cand cd = first_pass(t, A.mode == 2 ? 0.0f : amp);
         if (t < np) {
+            if (t < kFrKept) kept[threadIdx.x >> 5][t] = make_float2(dot, cd.d2raw);
             const float s = __fadd_rn(dot, cd.value);
             if (s > -1e10f) {
                 const unsigned long long key = make_key(s, (unsigned)t);
@@ -630,22 +652,47 @@ __global__ void __launch_bounds__(kFrWarps * 32, 3) max_frame_warp_kernel(const 
     // ---- second axis (compute_second_frame_each_edge.cu:81-142): per pair the arg-max over the translations of
     // a (d^2 - d^2_min) + log(max(1 - |cos|, 1e-5)) + noise among images with |cos| < 0.9999, the first translation in
     // the reference's loop order on equal values; the static variant's score is (d^2 - d^2_min) + log(...)
-    lead = warp_max_u64(lead);
-    const int seed_pair = (int)(0xFFFFFFFFu - (unsigned)(lead & 0xFFFFFFFFull));
+    // What the nearest images alone reach, less the noise (an image that beats its pair's nearest one with noise scores at most
+    // amp less without) and a margin for the fast arithmetic: pairs whose bound is below that cannot win, and the pair that
+    // reaches it is searched first.
     const float half = 0.5f * amp;
+    unsigned long long near = 0ull;
+    if (A.list != nullptr && a < 0.f && !A.is_static && (same_box || wider)) {
+        for (int t0 = 0; t0 < np; t0 += 32) {
+            const int t = t0 + lane;
+            if (np > 32) recall(t0, t);
+            if (t < np) {
+                const int64_t e = e0 + t;
+                const int code = __float_as_int(__ldg(A.list + (size_t)e * kListStride + 4 * kListLen));
+                place(e);
+                float dx, dy, dz, d2;
+                separation(cell, (float)((code & 255) - C), (float)(((code >> 8) & 255) - C), (float)(((code >> 16) & 255) - C), dx, dy, dz, d2);
+                const float cs = fabsf(dx * f1x + dy * f1y + dz * f1z) * rsqrtf(d2);
+                const float reached = dot + a * d2 + __logf(1.0f - cs) - amp - 1e-3f - 1e-5f * (fabsf(dot) + fabsf(a * d2));
+                if (d2 > 2e-5f && cs < 0.9998f && reached > -1e10f) {
+                    const unsigned long long key = make_key(reached, (unsigned)t);
+                    if (key > near) near = key;
+                }
+            }
+        }
+        near = warp_max_u64(near);
+    }
+    lead = near != 0ull ? near : warp_max_u64(lead);
+    const int seed_pair = (int)(0xFFFFFFFFu - (unsigned)(lead & 0xFFFFFFFFull));
     unsigned long long best2 = none;
+    auto threshold = [&]() { return max(order_of(best2), order_of(near)); };
     float wx = 0.f, wy = 0.f, wz = 0.f;                     // direction of the best pair's image
     int img2 = -1;
     for (int turn = 0; turn < 2 && np > 0; turn++) {        // the seed, then whatever can still win
         for (int t0 = turn == 0 ? seed_pair & ~31 : 0; t0 < np; t0 += 32) {
             const int t = t0 + lane;
-            if (np > 32) first_pass(t, 0.0f);               // one tile: still in registers
+            if (np > 32) recall(t0, t);
             unsigned todo = turn == 0 ? 1u << (seed_pair & 31)
-                                      : __ballot_sync(0xffffffffu, t < np && t != seed_pair && order_of(make_key(bound, 0u)) >= order_of(best2));
+                                      : __ballot_sync(0xffffffffu, t < np && t != seed_pair && order_of(make_key(bound, 0u)) >= threshold());
             while (todo) {
                 const int jj = __ffs(todo) - 1;
                 todo &= todo - 1;
-                if (turn == 1 && order_of(make_key(__shfl_sync(0xffffffffu, bound, jj), 0u)) < order_of(best2)) continue;
+                if (turn == 1 && order_of(make_key(__shfl_sync(0xffffffffu, bound, jj), 0u)) < threshold()) continue;
                 const int64_t e = e0 + t0 + jj;
                 const float dot_j = __shfl_sync(0xffffffffu, dot, jj), d2min = __shfl_sync(0xffffffffu, known, jj);
                 place(e);
@@ -1049,7 +1096,7 @@ int max_frame(const FrArgs& A, const Params& P, cudaStream_t st)
 {
     if (A.N == 0 || A.E == 0) return CFB200_OK;
     if (!A.is_static && !on_grid({A.q, A.k})) return CFB200_E_SHAPE;
-    if (A.E > kFrWarpPairs * A.N) {
+    if (A.E > (A.N * P.H >= kFrManyTasks ? kFrWarpPairs : kFrWarpPairsFew) * A.N) {
         max_frame_warp_kernel<<<(unsigned)((A.N * P.H + kFrWarps - 1) / kFrWarps), kFrWarps * 32, 0, st>>>(A, P);
         return cudaGetLastError() == cudaSuccess ? CFB200_OK : CFB200_E_CUDA;
     }
