@@ -311,6 +311,7 @@ __device__ __forceinline__ void fw_gaussians(const FwLane& L, const float4* R, c
 template <int AH, bool TASKS, int MODE>
 __global__ void __launch_bounds__(fw_warps(MODE) * 32, fw_blocks(MODE)) attn_tile_kernel(const AtArgs A, const Params P)
 {
+    wait_for_predecessors();
     extern __shared__ __align__(16) float smem[];
     constexpr int K = fw_k(AH), RS = kFwRec, kWarps = fw_warps(MODE);
     constexpr bool SAVE = MODE == 1, BACK = MODE == 2;
@@ -1018,6 +1019,7 @@ __device__ __forceinline__ void pairwise_task(const AtArgs& A, const Params& P, 
 template <bool ANG, bool TASKS>
 __global__ void __launch_bounds__(kPwWarps * 32, 2) attn_pairwise_kernel(const AtArgs A, const Params P)
 {
+    wait_for_predecessors();
     extern __shared__ __align__(16) float smem[];
     float* W_s = smem;                                      // [16][260]
     float* tbuf = W_s + kAtHd * kPwStride;                  // per warp 8 x 32
@@ -1119,6 +1121,7 @@ __device__ __noinline__ void ordered_slow_task(const AtArgs& A, const Params& P,
 template <bool TASKS>
 __global__ void __launch_bounds__(kOrWarps * 32, 2) attn_ordered_kernel(const __grid_constant__ AtArgs A, const __grid_constant__ Params P)
 {
+    wait_for_predecessors();
     extern __shared__ __align__(16) float smem[];
     float* W_s = smem;                                      // [16][kOrRow]
     const int H = P.H;
@@ -1433,6 +1436,7 @@ __device__ __forceinline__ float dot4(const float4 a, const float4 b) { return f
 
 __global__ void __launch_bounds__(kBsWarps * 32) attn_bwd_saved_kernel(const AtArgs A, const Params P)
 {
+    wait_for_predecessors();
     const int H = P.H, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int64_t i = blockIdx.x;
     const int head = blockIdx.y * 8 + (lane >> 2), h = min(head, H - 1);       // lanes beyond the last head repeat it
@@ -1508,6 +1512,7 @@ __global__ void __launch_bounds__(256) attn_plan_kernel(const int32_t* __restric
                                                         int64_t N, int64_t n_entries, int H, float scale, int* __restrict__ chunk_count,
                                                         int4* __restrict__ tasks)
 {
+    wait_for_predecessors();
     const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     const int h = blockIdx.y;
     if (t >= n_entries) return;
@@ -1543,6 +1548,7 @@ __global__ void __launch_bounds__(256) attn_plan_kernel(const int32_t* __restric
 // log-sum-exp over its own pairs; the whole is their average weighted by exp(lse_c - lse).
 __global__ void __launch_bounds__(256) attn_merge_fwd_kernel(const AtArgs A, const int H)
 {
+    wait_for_predecessors();
     const int lane = threadIdx.x & 31;
     const int64_t t = (int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
     const int h = blockIdx.y;
@@ -1580,6 +1586,7 @@ __global__ void __launch_bounds__(256) attn_merge_fwd_kernel(const AtArgs A, con
 // Backward: the chunks' parts of the query gradient and of the coefficient gradient are summed in chunk order.
 __global__ void __launch_bounds__(256) attn_merge_bwd_kernel(const AtArgs A, const int H)
 {
+    wait_for_predecessors();
     const int lane = threadIdx.x & 31;
     const int64_t t = (int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
     const int h = blockIdx.y;
@@ -1603,8 +1610,8 @@ int attn_plan(const int32_t* order, const int32_t* split, const float* a_ik, con
               int64_t n_entries, int H, float scale, int* chunk_count, int4* tasks, cudaStream_t st)
 {
     if (n_entries <= 0) return CFB200_OK;
-    attn_plan_kernel<<<dim3((unsigned)((n_entries + 255) / 256), H), 256, 0, st>>>(order, split, a_ik, e_start, N, n_entries, H, scale,
-                                                                                  chunk_count, tasks);
+    launch_ahead(attn_plan_kernel, dim3((unsigned)((n_entries + 255) / 256), H), 256, 0, st,
+                 order, split, a_ik, e_start, N, n_entries, H, scale, chunk_count, tasks);
     return cudaGetLastError() == cudaSuccess ? CFB200_OK : CFB200_E_CUDA;
 }
 
@@ -1620,11 +1627,12 @@ static int launch_tile(const AtArgs& A, const Params& P, cudaStream_t st)
         if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) return CFB200_E_CUDA;
         attr_done[dev & 63] = true;
     }
-    kern<<<dim3(at_grid_x(TASKS ? A.N * kSplitMaxChunks : A.N, P.H, MODE), P.H), fw_warps(MODE) * 32, smem, st>>>(A, P);
+    launch_ahead(kern, dim3(at_grid_x(TASKS ? A.N * kSplitMaxChunks : A.N, P.H, MODE), P.H), fw_warps(MODE) * 32, smem, st,
+                 A, P);
     if (TASKS) {
         const dim3 grid(kSplitSlots / 8, P.H);
-        if (MODE == 2) attn_merge_bwd_kernel<<<grid, 256, 0, st>>>(A, P.H);
-        else attn_merge_fwd_kernel<<<grid, 256, 0, st>>>(A, P.H);
+        if (MODE == 2) launch_ahead(attn_merge_bwd_kernel, grid, 256, 0, st, A, P.H);
+        else launch_ahead(attn_merge_fwd_kernel, grid, 256, 0, st, A, P.H);
     }
     return cudaGetLastError() == cudaSuccess ? CFB200_OK : CFB200_E_CUDA;
 }
@@ -1640,8 +1648,8 @@ static int launch_pairwise(const AtArgs& A, const Params& P, cudaStream_t st)
         if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kPwSmem) != cudaSuccess) return CFB200_E_CUDA;
         attr_done[dev & 63] = true;
     }
-    kern<<<dim3(pairwise_grid_x(A.N, P.H), P.H), kPwWarps * 32, kPwSmem, st>>>(A, P);
-    if (TASKS) attn_merge_fwd_kernel<<<dim3(kSplitSlots / 8, P.H), 256, 0, st>>>(A, P.H);
+    launch_ahead(kern, dim3(pairwise_grid_x(A.N, P.H), P.H), kPwWarps * 32, kPwSmem, st, A, P);
+    if (TASKS) launch_ahead(attn_merge_fwd_kernel, dim3(kSplitSlots / 8, P.H), 256, 0, st, A, P.H);
     return cudaGetLastError() == cudaSuccess ? CFB200_OK : CFB200_E_CUDA;
 }
 
@@ -1658,8 +1666,8 @@ static int launch_ordered(const AtArgs& A0, const Params& P, cudaStream_t st)
         if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kOrSmem) != cudaSuccess) return CFB200_E_CUDA;
         attr_done[dev & 63] = true;
     }
-    kern<<<dim3(pairwise_grid_x(A.N, P.H), P.H), kOrWarps * 32, kOrSmem, st>>>(A, P);
-    if (TASKS) attn_merge_fwd_kernel<<<dim3(kSplitSlots / 8, P.H), 256, 0, st>>>(A, P.H);
+    launch_ahead(kern, dim3(pairwise_grid_x(A.N, P.H), P.H), kOrWarps * 32, kOrSmem, st, A, P);
+    if (TASKS) launch_ahead(attn_merge_fwd_kernel, dim3(kSplitSlots / 8, P.H), 256, 0, st, A, P.H);
     return cudaGetLastError() == cudaSuccess ? CFB200_OK : CFB200_E_CUDA;
 }
 
@@ -1699,7 +1707,7 @@ int attn_fused_bwd(const AtArgs& A, const Params& P, cudaStream_t st)
     if (A.N == 0) return CFB200_OK;
     if (A.val == nullptr) return launch_tile<2>(A, P, st);
     if (!on_grid({A.qs, A.k, A.v, A.gout, A.out, A.upool, A.val, A.gq})) return CFB200_E_SHAPE;
-    attn_bwd_saved_kernel<<<dim3((unsigned)A.N, (unsigned)((P.H + 7) / 8)), kBsWarps * 32, 0, st>>>(A, P);
+    launch_ahead(attn_bwd_saved_kernel, dim3((unsigned)A.N, (unsigned)((P.H + 7) / 8)), kBsWarps * 32, 0, st, A, P);
     return cudaGetLastError() == cudaSuccess ? CFB200_OK : CFB200_E_CUDA;
 }
 

@@ -34,6 +34,7 @@ __device__ __forceinline__ float coef_from_dot(const CoefArgs& A, float dot, flo
 
 __global__ void __launch_bounds__(256) coef_fwd_kernel(const CoefArgs A)
 {
+    wait_for_predecessors();
     const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (t < A.H) {
         if (A.zero[0]) A.zero[0][t] = 0;
@@ -61,6 +62,7 @@ __global__ void __launch_bounds__(256) coef_fwd_kernel(const CoefArgs A)
 // slices in order by coef_bwd_reduce_kernel).
 __global__ void __launch_bounds__(256) coef_bwd_kernel(const CoefArgs A)
 {
+    wait_for_predecessors();
     __shared__ float part[256][kCoHd + 1];
     const int h = blockIdx.x, tid = threadIdx.x;
     const int64_t chunk = (A.N + gridDim.y - 1) / gridDim.y;
@@ -112,6 +114,7 @@ __global__ void __launch_bounds__(256) coef_bwd_kernel(const CoefArgs A)
 
 __global__ void coef_bwd_reduce_kernel(const CoefArgs A, int splits)
 {
+    wait_for_predecessors();
     const int t = blockIdx.x * blockDim.x + threadIdx.x;
     if (t >= A.H * kCoHd) return;
     float s = 0.f;
@@ -124,7 +127,7 @@ int coef_fwd(const CoefArgs& A, cudaStream_t st)
     const int64_t n = A.N * A.H;
     if (n == 0) return CFB200_OK;
     if (!on_grid({A.q, A.w, A.qs})) return CFB200_E_SHAPE;
-    coef_fwd_kernel<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(A);
+    launch_ahead(coef_fwd_kernel, (unsigned)((n + 255) / 256), 256, 0, st, A);
     return cudaGetLastError() == cudaSuccess ? CFB200_OK : CFB200_E_CUDA;
 }
 
@@ -132,10 +135,10 @@ int coef_bwd(const CoefArgs& A, cudaStream_t st)
 {
     if (!on_grid({A.q, A.gqs, A.gq})) return CFB200_E_SHAPE;
     if (A.partial != nullptr && A.N > 1024) {
-        coef_bwd_kernel<<<dim3(A.H, kCoSplits), 256, 0, st>>>(A);
-        coef_bwd_reduce_kernel<<<(A.H * kCoHd + 127) / 128, 128, 0, st>>>(A, kCoSplits);
+        launch_ahead(coef_bwd_kernel, dim3(A.H, kCoSplits), 256, 0, st, A);
+        launch_ahead(coef_bwd_reduce_kernel, (A.H * kCoHd + 127) / 128, 128, 0, st, A, kCoSplits);
     } else {
-        coef_bwd_kernel<<<dim3(A.H, 1), 256, 0, st>>>(A);
+        launch_ahead(coef_bwd_kernel, dim3(A.H, 1), 256, 0, st, A);
     }
     return cudaGetLastError() == cudaSuccess ? CFB200_OK : CFB200_E_CUDA;
 }

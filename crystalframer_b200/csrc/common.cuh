@@ -70,6 +70,30 @@ __device__ __forceinline__ float ex2_approx(float x)
     return y;
 }
 
+// Launches ahead: a kernel may be brought to the SMs while the last blocks of the one before it in the stream still run, and
+// waits there until everything before it has finished and its writes can be seen.  Every such kernel begins with that wait,
+// in all its blocks, before anything else that touches global memory; so a kernel that has finished has all its predecessors
+// behind it, as in any stream.  What it saves is the gap between two kernels, 1.7 us in a step of some 120 launches:
+// training step of 256 crystals 3.70 -> 3.52 ms, of 128 with the lightweight recipe 2.39 -> 2.19, prediction of 256
+// 2.21 -> 2.09.  (The weight gradients' kernels, the first behind a side stream's fork, are launched as usual.)
+__device__ __forceinline__ void wait_for_predecessors() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
+template <typename T> struct SameType { using type = T; };
+
+template <typename... K>
+inline cudaError_t launch_ahead(void (*kernel)(K...), const dim3 grid, const dim3 block, const size_t smem,
+                                const cudaStream_t st, typename SameType<K>::type... args)
+{
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid; cfg.blockDim = block; cfg.dynamicSmemBytes = smem; cfg.stream = st;
+    cudaLaunchAttribute attr = {};
+    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr.val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = &attr;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, kernel, args...);
+}
+
 // Packed FP32: two floats in one 64-bit register, one instruction for two fused multiply-adds (fma.rn.f32x2 and its
 // mul twin, sm_100).  Each half is an ordinary IEEE round-to-nearest operation; what is saved is issue slots.
 typedef unsigned long long f32x2;

@@ -54,6 +54,7 @@ __device__ __forceinline__ float dot16(const float* a, const float* b)
 
 __global__ void __launch_bounds__(kDpWarps * 32) dpa_fwd_kernel(const DpArgs A, int H, int Hs)
 {
+    wait_for_predecessors();
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int S = H / Hs;                                   // warps per atom
     const int64_t gw = (int64_t)blockIdx.x * kDpWarps + warp;
@@ -117,6 +118,7 @@ __global__ void __launch_bounds__(kDpWarps * 32) dpa_fwd_kernel(const DpArgs A, 
 //         gq_i = sum_j gz_ij * k_j           (fused_dpa_bwd.cu:52-124, fused_dpa_bwd_q.cu:27-52)
 __global__ void __launch_bounds__(kDpWarps * 32) dpa_bwd_rows_kernel(const DpArgs A, int H, int Hs)
 {
+    wait_for_predecessors();
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int S = H / Hs;                                   // warps per atom
     const int64_t gw = (int64_t)blockIdx.x * kDpWarps + warp;
@@ -171,6 +173,7 @@ __global__ void __launch_bounds__(kDpWarps * 32) dpa_bwd_rows_kernel(const DpArg
 // (i, j) has index e_start[i] + (j - a0).  gk_j = sum_i gz_ij q_i ; gv_j = sum_i p_ij gout_i.
 __global__ void __launch_bounds__(kDpWarps * 32) dpa_bwd_cols_kernel(const DpArgs A, int H, int Hs)
 {
+    wait_for_predecessors();
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int S = H / Hs;
     const int64_t gw = (int64_t)blockIdx.x * kDpWarps + warp;
@@ -228,7 +231,7 @@ int dpa_fwd(const DpArgs& A, const Params& P, cudaStream_t st)
     if (!on_grid({A.q, A.k, A.v, A.b, A.out})) return CFB200_E_SHAPE;
     const int Hs = heads_per_warp(P.H);
     const int64_t warps = A.N * (P.H / Hs);
-    dpa_fwd_kernel<<<(unsigned)((warps + kDpWarps - 1) / kDpWarps), kDpWarps * 32, 0, st>>>(A, P.H, Hs);
+    launch_ahead(dpa_fwd_kernel, (unsigned)((warps + kDpWarps - 1) / kDpWarps), kDpWarps * 32, 0, st, A, P.H, Hs);
     return cudaGetLastError() == cudaSuccess ? CFB200_OK : CFB200_E_CUDA;
 }
 
@@ -240,8 +243,8 @@ int dpa_bwd(const DpArgs& A, const Params& P, cudaStream_t st)
     const int Hs = heads_per_warp(P.H);
     const int64_t warps = A.N * (P.H / Hs);
     const unsigned grid = (unsigned)((warps + kDpWarps - 1) / kDpWarps);
-    dpa_bwd_rows_kernel<<<grid, kDpWarps * 32, 0, st>>>(A, P.H, Hs);
-    dpa_bwd_cols_kernel<<<grid, kDpWarps * 32, 0, st>>>(A, P.H, Hs);
+    launch_ahead(dpa_bwd_rows_kernel, grid, kDpWarps * 32, 0, st, A, P.H, Hs);
+    launch_ahead(dpa_bwd_cols_kernel, grid, kDpWarps * 32, 0, st, A, P.H, Hs);
     return cudaGetLastError() == cudaSuccess ? CFB200_OK : CFB200_E_CUDA;
 }
 
@@ -255,7 +258,7 @@ int dpa_bwd_cols(const DpArgs& A, const Params& P, cudaStream_t st)
     if (!dpa_cols_on_grid(A)) return CFB200_E_SHAPE;
     const int Hs = heads_per_warp(P.H);
     const int64_t warps = A.N * (P.H / Hs);
-    dpa_bwd_cols_kernel<<<(unsigned)((warps + kDpWarps - 1) / kDpWarps), kDpWarps * 32, 0, st>>>(A, P.H, Hs);
+    launch_ahead(dpa_bwd_cols_kernel, (unsigned)((warps + kDpWarps - 1) / kDpWarps), kDpWarps * 32, 0, st, A, P.H, Hs);
     return cudaGetLastError() == cudaSuccess ? CFB200_OK : CFB200_E_CUDA;
 }
 

@@ -77,6 +77,7 @@ __device__ __forceinline__ float2 fma2(float a0, float a1, float b0, float b1, f
 template <bool BWD, bool ANG>
 __global__ void __launch_bounds__(kFpThreads, fp_blocks_per_sm(BWD)) framed_proj_kernel(const FpArgs A, const Params P)
 {
+    wait_for_predecessors();
     extern __shared__ __align__(16) float smem[];
     constexpr int kFpStageStride = fp_stage_stride(BWD);
     constexpr int kFpSlots = fp_slots(BWD), kFpTasksPerWarp = fp_tasks_per_warp(BWD);
@@ -296,6 +297,7 @@ __global__ void __launch_bounds__(kFpThreads, fp_blocks_per_sm(BWD)) framed_proj
 __global__ void reduce_ga_kernel(const float* __restrict__ ga_e, const int64_t* __restrict__ e_start,
                                  int64_t N, int H, float* __restrict__ ga)
 {
+    wait_for_predecessors();
     const int64_t tid = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (tid >= N * H) return;
     const int64_t i = tid / H;
@@ -309,6 +311,7 @@ __global__ void reduce_ga_kernel(const float* __restrict__ ga_e, const int64_t* 
 __global__ void reduce_gw_kernel(const float* __restrict__ part, int nPart, int H, int angle_dim, float* gWd, float* gW1,
                                  float* gW2, float* gW3)
 {
+    wait_for_predecessors();
     const int tid = blockIdx.x * blockDim.x + threadIdx.x;   // (h, o, k)
     if (tid >= H * kHd * kFpK) return;
     float s = 0.f;
@@ -352,7 +355,7 @@ static int launch_fp(const FpArgs& A, const Params& P, int gx, cudaStream_t st)
             return CFB200_E_CUDA;
         attr_done[dev & 63] = true;
     }
-    kern<<<dim3(gx, P.H), kFpThreads, fp_smem_bytes(BWD), st>>>(A, P);
+    launch_ahead(kern, dim3(gx, P.H), kFpThreads, fp_smem_bytes(BWD), st, A, P);
     return cudaGetLastError() == cudaSuccess ? CFB200_OK : CFB200_E_CUDA;
 }
 
@@ -382,10 +385,11 @@ int framed_proj_bwd(FpArgs A, const Params& P, const int64_t* e_start, float* ga
     }
     if (A.N > 0) {
         const int64_t nt = A.N * P.H;
-        reduce_ga_kernel<<<(unsigned)((nt + 255) / 256), 256, 0, st>>>(A.ga_e, e_start, A.N, P.H, ga);
+        launch_ahead(reduce_ga_kernel, (unsigned)((nt + 255) / 256), 256, 0, st, A.ga_e, e_start, A.N, P.H, ga);
     }
     const int nw = P.H * kHd * kFpK;
-    reduce_gw_kernel<<<(nw + 255) / 256, 256, 0, st>>>(A.gW_part, nPart, P.H, P.angle_dim, gW[0], gW[1], gW[2], gW[3]);
+    launch_ahead(reduce_gw_kernel, (nw + 255) / 256, 256, 0, st,
+                 A.gW_part, nPart, P.H, P.angle_dim, gW[0], gW[1], gW[2], gW[3]);
     return cudaGetLastError() == cudaSuccess ? CFB200_OK : CFB200_E_CUDA;
 }
 

@@ -308,6 +308,7 @@ __device__ __forceinline__ int64_t lower_bound_i64(const int64_t* v, int64_t n, 
 
 __global__ void __launch_bounds__(kFrThreads, CFB_FR_BLOCKS) max_frame_kernel(const FrArgs A, const Params P)
 {
+    wait_for_predecessors();
     __shared__ unsigned long long best[kFrMaxRows];
     __shared__ long long row_start[kFrMaxRows + 1];
     __shared__ float row_a[kFrMaxRows];
@@ -527,6 +528,7 @@ constexpr int kFrKept = 256;
 
 __global__ void __launch_bounds__(kFrWarps * 32, 3) max_frame_warp_kernel(const FrArgs A, const Params P)
 {
+    wait_for_predecessors();
     __shared__ float2 kept[kFrWarps][kFrKept];
     const int H = P.H, lane = threadIdx.x & 31;
     const int64_t task = (int64_t)blockIdx.x * kFrWarps + (threadIdx.x >> 5);
@@ -820,6 +822,7 @@ __global__ void __launch_bounds__(128) lattice_frame_kernel(const float* __restr
                                                             float* __restrict__ f1, float* __restrict__ f2, float* __restrict__ f3,
                                                             const Params P)
 {
+    wait_for_predecessors();
     const int64_t tid = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     const int H = P.H;
     if (tid >= N * H) return;
@@ -902,6 +905,7 @@ __global__ void __launch_bounds__(256) pair_cache_kernel(const float* __restrict
                                                          const int64_t* __restrict__ batch, const int64_t* __restrict__ edges,
                                                          int64_t E, int R, float4* __restrict__ out)
 {
+    wait_for_predecessors();
     const int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (e >= E) return;
     const int64_t c = batch[edges[e]];
@@ -992,6 +996,7 @@ __global__ void __launch_bounds__(kPlWarps * 32) pair_list_kernel(const float* _
                                                                   const int64_t* __restrict__ batch, const int64_t* __restrict__ edges,
                                                                   int64_t E, int R, int vec, float* __restrict__ out)
 {
+    wait_for_predecessors();
     __shared__ float4 table[kListLen];                  // n1, n2, n3 and code of a translation
     const int lane = threadIdx.x & 31;
     const int L = 2 * R + 1, nT = L * L * L;
@@ -1071,12 +1076,12 @@ int pair_cache(const float* pos_ij, const float* tvecs, const int64_t* batch, co
 {
     if (E == 0) return CFB200_OK;
     if (out != nullptr)
-        pair_cache_kernel<<<(unsigned)((E + 255) / 256), 256, 0, st>>>(pos_ij, tvecs, batch, edges, E, R,
-                                                                      reinterpret_cast<float4*>(out));
+        launch_ahead(pair_cache_kernel, (unsigned)((E + 255) / 256), 256, 0, st,
+                     pos_ij, tvecs, batch, edges, E, R, reinterpret_cast<float4*>(out));
     if (list != nullptr) {
         if ((2 * R + 1) * (2 * R + 1) * (2 * R + 1) > kListLen) return CFB200_E_UNSUPPORTED;
-        pair_list_kernel<<<(unsigned)((E + kPlWarps * kPlPairs - 1) / (kPlWarps * kPlPairs)), kPlWarps * 32, 0, st>>>(pos_ij, tvecs, batch, edges, E, R,
-                                                                                                        on_grid({list}), list);
+        launch_ahead(pair_list_kernel, (unsigned)((E + kPlWarps * kPlPairs - 1) / (kPlWarps * kPlPairs)), kPlWarps * 32, 0, st,
+                     pos_ij, tvecs, batch, edges, E, R, on_grid({list}), list);
     }
     return cudaGetLastError() == cudaSuccess ? CFB200_OK : CFB200_E_CUDA;
 }
@@ -1087,8 +1092,8 @@ int lattice_frames(const float* a_ik, const float* tvecs, const float* rvlen, co
 {
     if (N == 0) return CFB200_OK;
     const int64_t n = N * P.H;
-    lattice_frame_kernel<<<(unsigned)((n + 127) / 128), 128, 0, st>>>(a_ik, tvecs, rvlen, batch, e_start, edges, N, E, seed1, seed2,
-                                                                    seed3, f1, f2, f3, P);
+    launch_ahead(lattice_frame_kernel, (unsigned)((n + 127) / 128), 128, 0, st,
+                 a_ik, tvecs, rvlen, batch, e_start, edges, N, E, seed1, seed2, seed3, f1, f2, f3, P);
     return cudaGetLastError() == cudaSuccess ? CFB200_OK : CFB200_E_CUDA;
 }
 
@@ -1097,11 +1102,11 @@ int max_frame(const FrArgs& A, const Params& P, cudaStream_t st)
     if (A.N == 0 || A.E == 0) return CFB200_OK;
     if (!A.is_static && !on_grid({A.q, A.k})) return CFB200_E_SHAPE;
     if (A.E > (A.N * P.H >= kFrManyTasks ? kFrWarpPairs : kFrWarpPairsFew) * A.N) {
-        max_frame_warp_kernel<<<(unsigned)((A.N * P.H + kFrWarps - 1) / kFrWarps), kFrWarps * 32, 0, st>>>(A, P);
+        launch_ahead(max_frame_warp_kernel, (unsigned)((A.N * P.H + kFrWarps - 1) / kFrWarps), kFrWarps * 32, 0, st, A, P);
         return cudaGetLastError() == cudaSuccess ? CFB200_OK : CFB200_E_CUDA;
     }
     const unsigned gx = (unsigned)((A.E + kFrPairs - 1) / kFrPairs);
-    max_frame_kernel<<<dim3(gx, P.H), kFrThreads, 0, st>>>(A, P);
+    launch_ahead(max_frame_kernel, dim3(gx, P.H), kFrThreads, 0, st, A, P);
     return cudaGetLastError() == cudaSuccess ? CFB200_OK : CFB200_E_CUDA;
 }
 
@@ -1123,6 +1128,7 @@ struct Fr3Args {
 
 __global__ void __launch_bounds__(256) third_axis_edges_kernel(const Fr3Args A, const Params P)
 {
+    wait_for_predecessors();
     const int H = P.H;
     const int64_t tid = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (tid >= A.E * H) return;
@@ -1186,6 +1192,7 @@ __global__ void __launch_bounds__(256) third_axis_edges_kernel(const Fr3Args A, 
 
 __global__ void __launch_bounds__(256) third_axis_select_kernel(const Fr3Args A, const Params P)
 {
+    wait_for_predecessors();
     const int H = P.H, lane = threadIdx.x & 31;
     const int64_t w = (int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
     if (w >= A.N * H) return;
@@ -1234,8 +1241,8 @@ int third_axis(const Fr3Args& A, const Params& P, cudaStream_t st)
     if (A.N == 0 || A.E == 0) return CFB200_OK;
     if (!on_grid({A.q, A.k})) return CFB200_E_SHAPE;
     const int64_t n1 = A.E * P.H, n2 = A.N * P.H;
-    third_axis_edges_kernel<<<(unsigned)((n1 + 255) / 256), 256, 0, st>>>(A, P);
-    third_axis_select_kernel<<<(unsigned)((n2 + 7) / 8), 256, 0, st>>>(A, P);
+    launch_ahead(third_axis_edges_kernel, (unsigned)((n1 + 255) / 256), 256, 0, st, A, P);
+    launch_ahead(third_axis_select_kernel, (unsigned)((n2 + 7) / 8), 256, 0, st, A, P);
     return cudaGetLastError() == cudaSuccess ? CFB200_OK : CFB200_E_CUDA;
 }
 

@@ -22,6 +22,7 @@ __global__ void __launch_bounds__(128) cell_kernel(const float* __restrict__ tve
                                                    float* __restrict__ vcell, float* __restrict__ key,
                                                    float* __restrict__ inv_vol)
 {
+    wait_for_predecessors();
     const int64_t c = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (c >= B) return;
     float m[9];
@@ -91,6 +92,7 @@ __global__ void __launch_bounds__(256) lattice_geometry_kernel(const float* __re
                                                                float* __restrict__ rvecs, float* __restrict__ vcell,
                                                                float* __restrict__ kr_base)
 {
+    wait_for_predecessors();
     const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (t < B) {
         const Reciprocal r = reciprocal_vectors(tvecs + 9 * t);
@@ -123,6 +125,7 @@ __global__ void __launch_bounds__(256) lattice_geometry_kernel(const float* __re
 __global__ void __launch_bounds__(256) pos_ij_kernel(const float* __restrict__ pos, const int64_t* __restrict__ edges, int64_t E,
                                                      float* __restrict__ pos_ij)
 {
+    wait_for_predecessors();
     const int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (e >= E) return;
     const int64_t i = edges[e], j = edges[E + e];
@@ -173,6 +176,7 @@ __global__ void __launch_bounds__(1024) atom_order_kernel(const float* __restric
                                                           int32_t* __restrict__ slot_of, int32_t* __restrict__ order,
                                                           int32_t* __restrict__ split)
 {
+    wait_for_predecessors();
     __shared__ int tmp[32];
     __shared__ int total;
     __shared__ float red[32];
@@ -384,8 +388,8 @@ int cfb200_lattice_geometry(const float* pos, const float* tvecs, const int64_t*
     if (n == 0) return CFB200_OK;
     if ((B > 0 && (!tvecs || !rvecs || !vcell)) || (E > 0 && (!pos || !edges || !pos_ij)) || (kr_base && E > 0 && !batch))
         return CFB200_E_NULL;
-    cfb::lattice_geometry_kernel<<<(unsigned)((n + 255) / 256), 256, 0, S(stream)>>>(pos, tvecs, batch, edges, B, N, E, pos_ij, rvecs,
-                                                                                   vcell, kr_base);
+    cfb::launch_ahead(cfb::lattice_geometry_kernel, (unsigned)((n + 255) / 256), 256, 0, S(stream),
+                      pos, tvecs, batch, edges, B, N, E, pos_ij, rvecs, vcell, kr_base);
     return cudaGetLastError() == cudaSuccess ? CFB200_OK : CFB200_E_CUDA;
 }
 
@@ -424,14 +428,15 @@ static int batch_geometry(const float* pos, const float* tvecs, const int64_t* s
     TmScope tm(CFB200_TM_GEOMETRY, st);
     int rc = cfb::edge_index(sizes, B, N, E, edges, e_start, batch, crystal_start, st);
     if (rc != CFB200_OK) return rc;
-    cfb::cell_kernel<<<(unsigned)((B + 127) / 128), 128, 0, st>>>(tvecs, sizes, B, rvecs, rvlen, vcell, key, inv_vol);
-    if (E > 0) cfb::pos_ij_kernel<<<(unsigned)((E + 255) / 256), 256, 0, st>>>(pos, edges, E, pos_ij);
+    cfb::launch_ahead(cfb::cell_kernel, (unsigned)((B + 127) / 128), 128, 0, st,
+                      tvecs, sizes, B, rvecs, rvlen, vcell, key, inv_vol);
+    if (E > 0) cfb::launch_ahead(cfb::pos_ij_kernel, (unsigned)((E + 255) / 256), 256, 0, st, pos, edges, E, pos_ij);
     // warps that serve one head's queue in the training forward, the launch the chunks are cut for
     const int heads = split != nullptr ? g_cfg.num_heads : 1;
     const int workers = pairwise ? cfb::pairwise_grid_x(N, heads) * cfb::kPwWarps : cfb::at_grid_x(N, heads, 1) * cfb::fw_warps(1);
-    cfb::atom_order_kernel<<<1, 1024, 0, st>>>(key, inv_vol, sizes, crystal_start, B, N, workers, pairwise ? 0.5f : 0.25f,
-                                               pairwise ? cfb::kSplitMinTargetPairwise : cfb::kSplitMinTarget, by_rank, start_of,
-                                               want_of, slot_of, order, split);
+    cfb::launch_ahead(cfb::atom_order_kernel, 1, 1024, 0, st,
+                      key, inv_vol, sizes, crystal_start, B, N, workers, pairwise ? 0.5f : 0.25f,
+                      pairwise ? cfb::kSplitMinTargetPairwise : cfb::kSplitMinTarget, by_rank, start_of, want_of, slot_of, order, split);
     if (cudaGetLastError() != cudaSuccess) return CFB200_E_CUDA;
     if (E > 0 && range > 0 && (pair_cache != nullptr || pair_list != nullptr)) {
         float* list = pair_list;

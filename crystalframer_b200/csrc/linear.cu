@@ -68,6 +68,7 @@ __device__ __forceinline__ void gemm_finish(const GemmArgs& G, const int m, cons
 template <bool B_KN, int TM>
 __global__ void __launch_bounds__(kGmThreads) gemm_kernel(const GemmBatch Gb)
 {
+    wait_for_predecessors();
     const GemmArgs& G = Gb.g[blockIdx.z / Gb.splits];
     constexpr int BM = 16 * TM;
     __shared__ __align__(16) float smem[4][kGmBK][kGmLd];
@@ -207,11 +208,13 @@ static int launch_gemm(GemmBatch& Gb, cudaStream_t st)
     cfg.gridDim = dim3(gx, gy, (unsigned)(Gb.n * Gb.splits));
     cfg.blockDim = dim3(kGmThreads);
     cfg.stream = st;
-    cudaLaunchAttribute attr = {};
-    attr.id = cudaLaunchAttributeClusterDimension;
-    attr.val.clusterDim.x = 1; attr.val.clusterDim.y = 1; attr.val.clusterDim.z = (unsigned)Gb.splits;
-    cfg.attrs = &attr;
-    cfg.numAttrs = Gb.splits > 1 ? 1 : 0;
+    cudaLaunchAttribute attr[2] = {};
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;      // as launch_ahead
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    attr[1].id = cudaLaunchAttributeClusterDimension;
+    attr[1].val.clusterDim.x = 1; attr[1].val.clusterDim.y = 1; attr[1].val.clusterDim.z = (unsigned)Gb.splits;
+    cfg.attrs = attr;
+    cfg.numAttrs = Gb.splits > 1 ? 2 : 1;
     return cudaLaunchKernelEx(&cfg, gemm_kernel<B_KN, TM>, (const GemmBatch)Gb) == cudaSuccess ? CFB200_OK : CFB200_E_CUDA;
 }
 
@@ -409,6 +412,7 @@ __global__ void __launch_bounds__(kGmThreads) wgrad_kernel(const WgArgs W)
 // grid.x covers the largest problem; grid.y = problem.  Sums the S partials of every output in split order.
 __global__ void __launch_bounds__(256) wgrad_reduce_kernel(const WgArgs W)
 {
+    wait_for_predecessors();
     const WgProblem& Pb = W.prob[blockIdx.y];
     const int64_t nW = (int64_t)Pb.nb * Pb.P * Pb.Q;
     const int64_t nAll = nW + (Pb.bias_out != nullptr ? Pb.P : 0);
@@ -491,7 +495,7 @@ static int wgrad(WgArgs& W, int64_t ws_floats, cudaStream_t st)
     if (fp.nprob > 0) wgrad_kernel<<<dim3(fp_tiles, W.S), kGmThreads, 0, st>>>(fp);
     int gx = (int)((largest + 255) / 256);
     if (gx > 148) gx = 148;
-    wgrad_reduce_kernel<<<dim3(gx, W.nprob), 256, 0, st>>>(W);
+    launch_ahead(wgrad_reduce_kernel, dim3(gx, W.nprob), 256, 0, st, W);
     return cudaGetLastError() == cudaSuccess ? CFB200_OK : CFB200_E_CUDA;
 }
 

@@ -24,6 +24,7 @@ constexpr int kOptThreads = 256;
 
 __global__ void __launch_bounds__(kOptThreads) grad_sumsq_kernel(const float* __restrict__ g, int64_t n, float* __restrict__ partial)
 {
+    wait_for_predecessors();
     __shared__ float red[kOptThreads];
     float s = 0.f;
     for (int64_t i = (int64_t)blockIdx.x * kOptThreads + threadIdx.x; i < n; i += (int64_t)kOptBlocks * kOptThreads) {
@@ -49,6 +50,7 @@ struct AdamArgs {
 
 __global__ void __launch_bounds__(kOptThreads) adamw_clip_kernel(const AdamArgs A)
 {
+    wait_for_predecessors();
     __shared__ float red[kOptThreads];
     red[threadIdx.x] = threadIdx.x < kOptBlocks ? A.partial[threadIdx.x] : 0.f;
     __syncthreads();
@@ -77,10 +79,10 @@ __global__ void __launch_bounds__(kOptThreads) adamw_clip_kernel(const AdamArgs 
 int adamw_clip_step(const AdamArgs& A, float* partial, cudaStream_t st)
 {
     if (A.n == 0) return CFB200_OK;
-    grad_sumsq_kernel<<<kOptBlocks, kOptThreads, 0, st>>>(A.g, A.n, partial);
+    launch_ahead(grad_sumsq_kernel, kOptBlocks, kOptThreads, 0, st, A.g, A.n, partial);
     int blocks = (int)((A.n + kOptThreads - 1) / kOptThreads);
     if (blocks > 1184) blocks = 1184;                       // 8 blocks per SM on 148 SMs
-    adamw_clip_kernel<<<blocks, kOptThreads, 0, st>>>(A);
+    launch_ahead(adamw_clip_kernel, blocks, kOptThreads, 0, st, A);
     return cudaGetLastError() == cudaSuccess ? CFB200_OK : CFB200_E_CUDA;
 }
 

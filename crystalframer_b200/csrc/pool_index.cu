@@ -12,6 +12,7 @@ __global__ void __launch_bounds__(1024) crystal_scan_kernel(const int64_t* __res
                                                             int64_t E, int64_t* __restrict__ crystal_start,
                                                             int64_t* __restrict__ e_start)
 {
+    wait_for_predecessors();
     __shared__ long long warp_a[32], warp_p[32];
     __shared__ long long carry_a, carry_p;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -62,6 +63,7 @@ __global__ void __launch_bounds__(256) edge_fill_kernel(const int64_t* __restric
                                                         int64_t N, int64_t E, int64_t* __restrict__ edges,
                                                         int64_t* __restrict__ e_start, int64_t* __restrict__ batch)
 {
+    wait_for_predecessors();
     for (int64_t c = blockIdx.x; c < B; c += gridDim.x) {
         const int64_t n = sizes[c], a0 = crystal_start[c];
         if (n <= 0 || a0 + n > N) continue;
@@ -83,6 +85,7 @@ __global__ void __launch_bounds__(256) edge_fill_kernel(const int64_t* __restric
 // e_start from a pair list sorted by query atom: e_start[i] = first pair whose query atom is >= i
 __global__ void csr_offsets_kernel(const int64_t* __restrict__ edge_i, int64_t E, int64_t N, int64_t* __restrict__ e_start)
 {
+    wait_for_predecessors();
     const int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (e > E) return;
     const int64_t prev = e == 0 ? -1 : edge_i[e - 1];
@@ -95,6 +98,7 @@ __global__ void csr_offsets_kernel(const int64_t* __restrict__ edge_i, int64_t E
 __global__ void __launch_bounds__(128) segment_mean_fwd_kernel(const float* __restrict__ x, const int64_t* __restrict__ start,
                                                                int64_t B, int64_t D, float* __restrict__ out)
 {
+    wait_for_predecessors();
     const int64_t groups = (D + 31) / 32;
     const int64_t task = (int64_t)blockIdx.x * 4 + (threadIdx.x >> 5);
     if (task >= B * groups) return;
@@ -113,6 +117,7 @@ __global__ void __launch_bounds__(128) segment_mean_fwd_kernel(const float* __re
 __global__ void __launch_bounds__(128) segment_mean_bwd_kernel(const float* __restrict__ gout, const int64_t* __restrict__ start,
                                                                int64_t B, int64_t D, float* __restrict__ gx)
 {
+    wait_for_predecessors();
     const int64_t groups = (D + 31) / 32;
     const int64_t task = (int64_t)blockIdx.x * 4 + (threadIdx.x >> 5);
     if (task >= B * groups) return;
@@ -126,17 +131,17 @@ __global__ void __launch_bounds__(128) segment_mean_bwd_kernel(const float* __re
 int edge_index(const int64_t* sizes, int64_t B, int64_t N, int64_t E, int64_t* edges, int64_t* e_start, int64_t* batch,
                int64_t* crystal_start, cudaStream_t st)
 {
-    crystal_scan_kernel<<<1, 1024, 0, st>>>(sizes, B, N, E, crystal_start, e_start);
+    launch_ahead(crystal_scan_kernel, 1, 1024, 0, st, sizes, B, N, E, crystal_start, e_start);
     if (B > 0) {
         const unsigned grid = (unsigned)(B < 65535 ? B : 65535);
-        edge_fill_kernel<<<grid, 256, 0, st>>>(sizes, crystal_start, B, N, E, edges, e_start, batch);
+        launch_ahead(edge_fill_kernel, grid, 256, 0, st, sizes, crystal_start, B, N, E, edges, e_start, batch);
     }
     return cudaGetLastError() == cudaSuccess ? CFB200_OK : CFB200_E_CUDA;
 }
 
 int csr_offsets(const int64_t* edge_i, int64_t E, int64_t N, int64_t* e_start, cudaStream_t st)
 {
-    csr_offsets_kernel<<<(unsigned)((E + 1 + 255) / 256), 256, 0, st>>>(edge_i, E, N, e_start);
+    launch_ahead(csr_offsets_kernel, (unsigned)((E + 1 + 255) / 256), 256, 0, st, edge_i, E, N, e_start);
     return cudaGetLastError() == cudaSuccess ? CFB200_OK : CFB200_E_CUDA;
 }
 
@@ -145,8 +150,8 @@ int segment_mean(bool bwd, const float* in, const int64_t* start, int64_t B, int
     const int64_t tasks = B * ((D + 31) / 32);
     if (tasks == 0) return CFB200_OK;
     const unsigned grid = (unsigned)((tasks + 3) / 4);
-    if (bwd) segment_mean_bwd_kernel<<<grid, 128, 0, st>>>(in, start, B, D, out);
-    else segment_mean_fwd_kernel<<<grid, 128, 0, st>>>(in, start, B, D, out);
+    if (bwd) launch_ahead(segment_mean_bwd_kernel, grid, 128, 0, st, in, start, B, D, out);
+    else launch_ahead(segment_mean_fwd_kernel, grid, 128, 0, st, in, start, B, D, out);
     return cudaGetLastError() == cudaSuccess ? CFB200_OK : CFB200_E_CUDA;
 }
 

@@ -28,6 +28,7 @@ struct ReciArgs {
 template <bool BWD>
 __global__ void __launch_bounds__(kReciWarps * 32) reci_enc_kernel(const ReciArgs A)
 {
+    wait_for_predecessors();
     extern __shared__ __align__(16) float reci_table[];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int i = blockIdx.x * kReciWarps + warp;
@@ -111,8 +112,8 @@ int reci_enc(const ReciArgs& A, bool bwd, cudaStream_t st)
     const int w = 2 * A.R + 1;
     const size_t smem = (size_t)kReciWarps * (A.R + 1) * w * w * kReciHeads * sizeof(float);
     const int blocks = (A.N + kReciWarps - 1) / kReciWarps;
-    if (bwd) reci_enc_kernel<true><<<blocks, kReciWarps * 32, smem, st>>>(A);
-    else reci_enc_kernel<false><<<blocks, kReciWarps * 32, smem, st>>>(A);
+    if (bwd) launch_ahead(reci_enc_kernel<true>, blocks, kReciWarps * 32, smem, st, A);
+    else launch_ahead(reci_enc_kernel<false>, blocks, kReciWarps * 32, smem, st, A);
     return cudaGetLastError() == cudaSuccess ? CFB200_OK : CFB200_E_CUDA;
 }
 

@@ -84,6 +84,7 @@ __device__ void sigma_pair_sweep(const SgArgs& A, const Params& P, const int64_t
 // thread = (pair, head): every pair by the sweep (no sorted lists at hand, or a head count that does not divide 32)
 __global__ void __launch_bounds__(256) sigma_edges_kernel(const SgArgs A, const Params P)
 {
+    wait_for_predecessors();
     const int64_t tid = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     const int H = P.H;
     if (tid >= A.E * H) return;
@@ -107,6 +108,7 @@ constexpr int kSgListWarps = 8;
 
 __global__ void __launch_bounds__(kSgListWarps * 32) sigma_edges_list_kernel(const SgArgs A, const Params P)
 {
+    wait_for_predecessors();
     const int H = P.H, lane = threadIdx.x & 31;
     const int64_t e = (int64_t)blockIdx.x * kSgListWarps + (threadIdx.x >> 5);
     if (e >= A.E) return;
@@ -288,6 +290,7 @@ __device__ void eigh3(float M[3][3], float w[3], float V[3][3])
 // warp = (atom, head): attention pooling of the pairs' moments, then the frame
 __global__ void __launch_bounds__(128) sigma_frames_kernel(const SgArgs A, const Params P)
 {
+    wait_for_predecessors();
     const int lane = threadIdx.x & 31;
     const int64_t task = (int64_t)blockIdx.x * 4 + (threadIdx.x >> 5);
     const int H = P.H;
@@ -379,6 +382,7 @@ __global__ void __launch_bounds__(128) pca_frames_kernel(const float* __restrict
                                                          int64_t N, int H, uint64_t seed, float* __restrict__ f1,
                                                          float* __restrict__ f2, float* __restrict__ f3)
 {
+    wait_for_predecessors();
     const int lane = threadIdx.x & 31;
     const int64_t i = (int64_t)blockIdx.x * 4 + (threadIdx.x >> 5);
     if (i >= N) return;
@@ -421,17 +425,18 @@ int pca_frames(const float* pos_ij, const int64_t* e_start, int64_t N, int H, ui
                cudaStream_t st)
 {
     if (N == 0) return CFB200_OK;
-    pca_frames_kernel<<<(unsigned)((N + 3) / 4), 128, 0, st>>>(pos_ij, e_start, N, H, seed, f1, f2, f3);
+    launch_ahead(pca_frames_kernel, (unsigned)((N + 3) / 4), 128, 0, st, pos_ij, e_start, N, H, seed, f1, f2, f3);
     return cudaGetLastError() == cudaSuccess ? CFB200_OK : CFB200_E_CUDA;
 }
 
 static void launch_sigma_edges(const SgArgs& A, const Params& P, cudaStream_t st)
 {
     if (A.list != nullptr && P.H <= 32 && 32 % P.H == 0) {
-        sigma_edges_list_kernel<<<(unsigned)((A.E + kSgListWarps - 1) / kSgListWarps), kSgListWarps * 32, 0, st>>>(A, P);
+        launch_ahead(sigma_edges_list_kernel, (unsigned)((A.E + kSgListWarps - 1) / kSgListWarps), kSgListWarps * 32, 0, st,
+                     A, P);
     } else {
         const int64_t n1 = A.E * P.H;
-        sigma_edges_kernel<<<(unsigned)((n1 + 255) / 256), 256, 0, st>>>(A, P);
+        launch_ahead(sigma_edges_kernel, (unsigned)((n1 + 255) / 256), 256, 0, st, A, P);
     }
 }
 
@@ -449,7 +454,7 @@ int sigma_frames(const SgArgs& A, const Params& P, cudaStream_t st)
     if (!on_grid({A.q, A.k})) return CFB200_E_SHAPE;
     launch_sigma_edges(A, P, st);
     const int64_t n2 = A.N * P.H;
-    sigma_frames_kernel<<<(unsigned)((n2 + 3) / 4), 128, 0, st>>>(A, P);
+    launch_ahead(sigma_frames_kernel, (unsigned)((n2 + 3) / 4), 128, 0, st, A, P);
     return cudaGetLastError() == cudaSuccess ? CFB200_OK : CFB200_E_CUDA;
 }
 

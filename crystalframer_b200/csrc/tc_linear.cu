@@ -363,9 +363,10 @@ __global__ void __launch_bounds__(kTcBlock, 2) tc_gemm_kernel(const GemmBatch Gb
     };
     TcSlice R0, R1;
     const bool brings = threadIdx.x < kTcThreads;
-    if (brings) { fetch(R0); fetch(R1); }
     TcCta T;
     tc_begin(T, tc_smem, mbar_slots, &tmem_slot);
+    wait_for_predecessors();
+    if (brings) { fetch(R0); fetch(R1); }
     if (brings) {
         for (int s = 0; s < total; s += 2) {
             tc_slice<false, B_KN>(T, R0); fetch(R0);
@@ -450,11 +451,13 @@ static int launch_tc_gemm(GemmBatch& Gb, cudaStream_t st)
     cfg.blockDim = dim3(kTcBlock);
     cfg.dynamicSmemBytes = kTcSmemBytes;
     cfg.stream = st;
-    cudaLaunchAttribute attr = {};
-    attr.id = cudaLaunchAttributeClusterDimension;
-    attr.val.clusterDim.x = 1; attr.val.clusterDim.y = 1; attr.val.clusterDim.z = (unsigned)Gb.splits;
-    cfg.attrs = &attr;
-    cfg.numAttrs = Gb.splits > 1 ? 1 : 0;
+    cudaLaunchAttribute attr[2] = {};
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;      // as launch_ahead
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    attr[1].id = cudaLaunchAttributeClusterDimension;
+    attr[1].val.clusterDim.x = 1; attr[1].val.clusterDim.y = 1; attr[1].val.clusterDim.z = (unsigned)Gb.splits;
+    cfg.attrs = attr;
+    cfg.numAttrs = Gb.splits > 1 ? 2 : 1;
     return cudaLaunchKernelEx(&cfg, kern, (const GemmBatch)Gb) == cudaSuccess ? CFB200_OK : CFB200_E_CUDA;
 }
 

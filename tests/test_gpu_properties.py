@@ -524,3 +524,38 @@ def test_translation_lists_are_sorted(sizes, rng, offset):
     xyz = got[:, 1:4, :nT].permute(0, 2, 1).double()
     assert ((xyz - want).abs() <= 4 * 2.0 ** -24 * 40.0).all()              # three fused steps on numbers below 40
     assert ((d2.double() - xyz.square().sum(-1)).abs() <= 3 * 2.0 ** -24 * xyz.square().sum(-1)).all()
+
+
+@pytest.mark.parametrize("method", ["max", "no", "weighted_pca"])
+def test_prediction_in_a_captured_graph(method):
+    """Kernels launched ahead of their predecessors' end keep their order in a captured graph: replays give the eager
+    prediction bit for bit, also on inputs that a kernel wrote just before."""
+    if not torch.cuda.is_available():
+        pytest.skip("no CUDA device")
+    from crystalframer_b200 import data, synth
+    from crystalframer_b200.latticeformer import Latticeformer, ModelParams
+    dev = torch.device("cuda:0")
+    torch.manual_seed(0)
+    model = Latticeformer(ModelParams(num_layers=2, frame_method=method, value_pe_angle_real=0 if method == "no" else 64)).to(dev).train()
+    tb = data.host_batch(synth.make_batch(48, 5), np.zeros((48, 1), np.float32), pinned=False).to(dev, non_blocking=False)
+    with torch.no_grad():
+        model(tb)
+    model.eval()
+
+    def predict():
+        np.random.seed(3)
+        torch.manual_seed(3)
+        with torch.no_grad():
+            return model(tb)
+    side = torch.cuda.Stream()
+    with torch.cuda.stream(side):
+        want = predict()
+    side.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        got = predict()
+    for _ in range(3):
+        tb.pos.copy_(tb.pos.clone())
+        graph.replay()
+        torch.cuda.synchronize()
+        assert torch.equal(got, want)
