@@ -43,6 +43,14 @@ def f32c(t):
     return t.clone() if t.data_ptr() & 15 else t
 
 
+def stamp(*tensors):
+    """What a result that is kept for these tensors is compared by: where their memory is and how it is read, and the version
+    of its contents (none that could ever be equal for tensors that do not count theirs).  It holds as long as whoever keeps it
+    also keeps the tensors, or aliases of them: else another tensor could come to lie at the address."""
+    return tuple(None if t is None else (t.data_ptr(), object() if t.is_inference() else t._version, t.shape, t.stride(), t.dtype)
+                 for t in tensors)
+
+
 _pair_cache = {}
 PAIR_LIST_BYTES_PER_PAIR = 5 * 128 * 4   # five planes of 128 floats: 2.5 KB of translation list per pair
 PAIR_LIST_MAX_PAIRS = 4_000_000          # hard cap (10 GB); below it the list also has to fit a quarter of the free memory
@@ -86,8 +94,8 @@ def pair_geometry(rpos_ij_e, tvecs_n, batch_i, edge_ij_e, cutoff):
     """(pair_cache, pair_list, cache_range): which lattice translations of every pair are near, and how
     near -- the nearest non-zero image, the smallest squared distance, all translations sorted by distance.
     Pure geometry, identical for every head and layer, so it is computed on the first call that sees a
-    batch's relative positions and kept while that tensor is alive and unmodified; the reference redoes
-    this search inside every kernel launch.  Returns (None, None, 0) when no range can be fixed up front."""
+    batch's relative positions and kept while that tensor is alive and it, the cells, the atoms' crystals and
+    the pair list are what they were; the reference redoes this search inside every kernel launch.  Returns (None, None, 0) when no range can be fixed up front."""
     from .kernel_manager import KernelManager
     cfg = KernelManager.config
     if cfg is None or rpos_ij_e is None or edge_ij_e.shape[1] == 0:
@@ -96,7 +104,7 @@ def pair_geometry(rpos_ij_e, tvecs_n, batch_i, edge_ij_e, cutoff):
     if rng <= 0:
         return None, None, 0
     key = id(rpos_ij_e)
-    sig = (rpos_ij_e._version, rpos_ij_e.data_ptr(), tvecs_n.data_ptr(), tvecs_n._version, edge_ij_e.data_ptr(), rng)
+    sig = (rng, stamp(rpos_ij_e, tvecs_n, batch_i, edge_ij_e))
     hit = _pair_cache.get(key)
     if hit is not None and hit[0]() is rpos_ij_e and hit[1] == sig:
         return hit[2], hit[3], rng
@@ -113,5 +121,5 @@ def pair_geometry(rpos_ij_e, tvecs_n, batch_i, edge_ij_e, cutoff):
                 _lib.ptr(cache), _lib.ptr(plist))
     for k in [k for k, v in _pair_cache.items() if v[0]() is None]:      # lists are large: drop dead batches at once
         del _pair_cache[k]
-    _pair_cache[key] = (weakref.ref(rpos_ij_e), sig, cache, plist)
+    _pair_cache[key] = (weakref.ref(rpos_ij_e), sig, cache, plist, tvecs_n.detach(), batch_i.detach(), edge_ij_e.detach())
     return cache, plist, rng

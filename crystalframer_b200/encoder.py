@@ -17,6 +17,8 @@ from . import _lib
 from . import fused_layer
 from .attention import CrystalformerMultiheadAttentionCUDA, gauss_scale_ready
 from .cuda_funcs import compile_kernels, register_csr
+from .cuda_funcs.common import stamp
+from .cuda_funcs.kernel_manager import KernelManager
 from .latticeformer_params import LatticeformerParams
 
 
@@ -175,11 +177,17 @@ class CrystalformerEncoderLayerCUDA(Module):
         meta = self.fused_meta(x)
         if meta is None:
             return None
+        # the layers of a batch share its geometry, which hangs on the pair list; any other tensor may have been exchanged or
+        # written to since
+        cfg = KernelManager.config
+        sig = (meta["cutoff"], cfg and (cfg.lattice_range, cfg.minimum_range), stamp(pos_ij, trans, batch, edges, rvecs))
         geo = getattr(edges, "_cf_geometry", None)
-        if geo is None or geo.pos_ij is not pos_ij:
+        if geo is None or geo.made_from != sig:
             rvlen = torch.norm(rvecs, 2, dim=-1).contiguous() if meta["cutoff"] != 0.0 else None
             geo = fused_layer.LayerGeometry.from_tensors(pos_ij.contiguous(), trans.contiguous(), batch.contiguous(),
                                                          edges.contiguous(), rvlen, meta["cutoff"])
+            geo.made_from = sig
+            geo._keep += [t.detach() for t in (pos_ij, trans, batch, rvecs)]        # the stamp's addresses stay theirs
             edges._cf_geometry = geo
         return self.fused_apply(x, geo, meta)
 

@@ -483,6 +483,55 @@ def test_layers_called_with_tensors_leave_no_memory_behind():
     assert last - first < 1 << 20, (first, last)            # a batch's lists alone: some 5 MB
 
 
+@pytest.mark.parametrize("change", ["cells written", "other cells", "positions written", "crystals written", "lengths written"])
+@pytest.mark.parametrize("path", ["layer", "frames"])
+def test_geometry_kept_for_a_batch_follows_its_tensors(change, path):
+    """A layer, or the drop-in frames, called again with one of a batch's tensors written to or exchanged (a new tensor in the
+    place in memory that the old one left) gives what a call with copies of all of them gives."""
+    if not torch.cuda.is_available():
+        pytest.skip("no CUDA device")
+    from crystalframer_b200 import cuda_funcs as F, data, synth
+    from crystalframer_b200.encoder import compute_lattice_distances_for_cuda
+    from crystalframer_b200.latticeformer import Latticeformer, ModelParams
+    dev = torch.device("cuda:0")
+    torch.manual_seed(1)
+    model = Latticeformer(ModelParams(num_layers=1, symm_break_noise=0.0)).to(dev).train()
+    tb = data.host_batch(synth.make_batch(16, 3, size_dist="uniform", size_lo=6, size_hi=6), np.zeros((16, 1), np.float32),
+                         pinned=False).to(dev, non_blocking=False)
+    with torch.no_grad():
+        model(tb)
+    layer, x = model.encoder.layers[0].eval(), model.input_embeddings(tb.x).detach()
+    pos_ij, _, _, rvecs, _, edges = compute_lattice_distances_for_cuda(tb.pos, tb.batch, tb.trans_vec, tb.sizes, 2, output_real=True)
+    cells, batch = tb.trans_vec.clone(), tb.batch.clone()
+    g = torch.Generator().manual_seed(2)
+    q, k = (torch.randn(len(x), 8, 16, generator=g).to(dev) for _ in range(2))
+    a = torch.full((len(x), 8), -0.25, device=dev)
+
+    def call(pos_ij, cells, rvecs, batch, edges):
+        with torch.no_grad():
+            if path == "layer":
+                return layer(x, batch, edges, pos_ij, None, cells, None, rvecs, None)
+            return torch.stack(F.max_frames_fused(q, k, a, pos_ij, cells, batch, edges, torch.norm(rvecs, 2, dim=-1), -3.5))
+    first = call(pos_ij, cells, rvecs, batch, edges)
+    if change == "cells written":
+        cells.copy_(cells.flip(0))
+    elif change == "other cells":
+        new, at = cells.flip(0).cpu(), cells.data_ptr()
+        del cells
+        cells = torch.empty(16, 3, 3, device=dev)
+        assert path != "frames" or cells.data_ptr() != at            # kept with what was made from them
+        cells = new.to(dev)
+    elif change == "positions written":
+        pos_ij.mul_(0.9)
+    elif change == "crystals written":
+        batch.copy_(15 - batch)
+    else:
+        rvecs.mul_(3.0)
+    got = call(pos_ij, cells, rvecs, batch, edges)
+    assert torch.equal(got, call(*(t.clone() for t in (pos_ij, cells, rvecs, batch, edges))))
+    assert change == "lengths written" or not torch.equal(got, first)
+
+
 @pytest.mark.parametrize("sizes", [(1,), (5, 2, 1, 1, 1), (1, 4, 4), (7, 9, 3)])        # 1, 32, 33 and 139 pairs
 @pytest.mark.parametrize("rng", [1, 2])
 @pytest.mark.parametrize("offset", [0, 1])
