@@ -287,6 +287,23 @@ __device__ __forceinline__ float box_reach2(const Cell& c, const int C)
     return r > 0.f ? r * r * 0.999f : 0.f;
 }
 
+// A score that a pair with q.k = dot is certain to reach on the second axis: that of its nearest image, number `code` of the
+// box (C)^3, less the noise (an image that beats it with noise scores at most amp less without).  In fast arithmetic, rounded
+// down: |cos| differs from the search's by less than 1e-6 of the sizes of its three terms (some ten roundings of 2^-24 and the
+// 2 ulp of rsqrtf), which is 5e-3 of 1 - |cos| next to the axis and any number for a first axis that is not of unit length;
+// what that leaves of 1 - |cos| is used.  The last two terms cover the logarithm and the rounding of the sums.  -1e15 where the
+// search might not take the image.
+__device__ __forceinline__ float certain_score(const Cell& cell, const int code, const int C, const float a, const float dot,
+                                               const float amp, const float f1x, const float f1y, const float f1z)
+{
+    float dx, dy, dz, d2;
+    separation(cell, (float)((code & 255) - C), (float)(((code >> 8) & 255) - C), (float)(((code >> 16) & 255) - C), dx, dy, dz, d2);
+    const float x = dx * f1x, y = dy * f1y, z = dz * f1z, rinv = rsqrtf(d2);
+    const float open = 1.0f - (fabsf(x + y + z) + 1e-6f * (fabsf(x) + fabsf(y) + fabsf(z))) * rinv;
+    if (!(d2 > 2e-5f && open > 2e-4f)) return -1e15f;
+    return dot + a * d2 + __logf(open) - amp - 1e-3f - 1e-5f * (fabsf(dot) + fabsf(a * d2));
+}
+
 // (score, pair) -> 64-bit key whose unsigned order is (score ascending, pair index descending)
 __device__ __forceinline__ unsigned long long make_key(float score, unsigned local_pair)
 {
@@ -430,10 +447,10 @@ __global__ void __launch_bounds__(kFrThreads, CFB_FR_BLOCKS) max_frame_kernel(co
                     // (the static search runs farthest-first, so it needs the list of the task's whole box)
                     hit = A.list != nullptr && (same_box || (!A.is_static && wider && reach2 > 0.f));
                     d2_known = known; reach2_known = reach2; dot_kept = dot;
-                    // What the pair's nearest image alone reaches, less the noise (an image that beats it with noise scores at
-                    // most the amplitude less without) and a margin for the fast arithmetic; and the bound on its score.  Pairs
-                    // whose bound is below what any pair of the atom reaches can neither win nor tie and are not searched: the
-                    // block waits for its slowest search (256 log-normal crystals 98 -> 84 us per launch, 1 024 304 -> 269).
+                    // What the pair is certain to reach, and the bound on its score.  Pairs whose bound is below what any pair of
+                    // the atom reaches can neither win nor tie and are not searched: the block waits for its slowest search.  Per
+                    // launch, without / with it: 256 log-normal crystals 100 / 85 us, 1 024 297 / 262, 256 crystals of 4-16 atoms
+                    // 93 / 85, 1 024 218 / 175, 256 of 1-4 atoms 47 / 46.
                     const float a = row_a[r];
                     bound = 0xffffffffu;
                     if (a < 0.f && !A.is_static && known >= 0.f) {
@@ -441,12 +458,8 @@ __global__ void __launch_bounds__(kFrThreads, CFB_FR_BLOCKS) max_frame_kernel(co
                         bound = (unsigned)(make_key(dot + g + 1e-6f * (fabsf(dot) + fabsf(g)), 0u) >> 32);
                         if (A.list != nullptr && (same_box || wider)) {
                             const int code = __float_as_int(__ldg(A.list + (size_t)e * kListStride + 4 * kListLen));
-                            float dx, dy, dz, d2;
-                            separation(cell, (float)((code & 255) - C), (float)(((code >> 8) & 255) - C),
-                                       (float)(((code >> 16) & 255) - C), dx, dy, dz, d2);
-                            const float cs = fabsf(dx * row_f1[r][0] + dy * row_f1[r][1] + dz * row_f1[r][2]) * rsqrtf(d2);
-                            const float reached = dot + a * d2 + __logf(1.0f - cs) - P.noise - 1e-3f - 1e-5f * (fabsf(dot) + fabsf(a * d2));
-                            if (d2 > 2e-5f && cs < 0.9998f && reached > -1e10f) atomicMax(&row_near[r], (unsigned)(make_key(reached, 0u) >> 32));
+                            const float reached = certain_score(cell, code, C, a, dot, P.noise, row_f1[r][0], row_f1[r][1], row_f1[r][2]);
+                            if (reached > -1e10f) atomicMax(&row_near[r], (unsigned)(make_key(reached, 0u) >> 32));
                         }
                     }
                 }
@@ -687,9 +700,8 @@ __global__ void __launch_bounds__(kFrWarps * 32, 3) max_frame_warp_kernel(const 
     // ---- second axis (compute_second_frame_each_edge.cu:81-142): per pair the arg-max over the translations of
     // a (d^2 - d^2_min) + log(max(1 - |cos|, 1e-5)) + noise among images with |cos| < 0.9999, the first translation in
     // the reference's loop order on equal values; the static variant's score is (d^2 - d^2_min) + log(...)
-    // What the nearest images alone reach, less the noise (an image that beats its pair's nearest one with noise scores at most
-    // amp less without) and a margin for the fast arithmetic: pairs whose bound is below that cannot win, and the pair that
-    // reaches it is searched first.
+    // Pairs whose bound is below what the nearest images are certain to reach cannot win, and the pair that reaches it is
+    // searched first.
     const float half = 0.5f * amp;
     unsigned long long near = 0ull;
     if (A.list != nullptr && a < 0.f && !A.is_static && (same_box || wider)) {
@@ -700,11 +712,8 @@ __global__ void __launch_bounds__(kFrWarps * 32, 3) max_frame_warp_kernel(const 
                 const int64_t e = e0 + t;
                 const int code = __float_as_int(__ldg(A.list + (size_t)e * kListStride + 4 * kListLen));
                 place(e);
-                float dx, dy, dz, d2;
-                separation(cell, (float)((code & 255) - C), (float)(((code >> 8) & 255) - C), (float)(((code >> 16) & 255) - C), dx, dy, dz, d2);
-                const float cs = fabsf(dx * f1x + dy * f1y + dz * f1z) * rsqrtf(d2);
-                const float reached = dot + a * d2 + __logf(1.0f - cs) - amp - 1e-3f - 1e-5f * (fabsf(dot) + fabsf(a * d2));
-                if (d2 > 2e-5f && cs < 0.9998f && reached > -1e10f) {
+                const float reached = certain_score(cell, code, C, a, dot, amp, f1x, f1y, f1z);
+                if (reached > -1e10f) {
                     const unsigned long long key = make_key(reached, (unsigned)t);
                     if (key > near) near = key;
                 }

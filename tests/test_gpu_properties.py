@@ -532,6 +532,69 @@ def test_geometry_kept_for_a_batch_follows_its_tensors(change, path):
     assert change == "lengths written" or not torch.equal(got, first)
 
 
+def _close_second_axis(B, atoms, length, rng):
+    """B cells of ``atoms`` atoms: seen from its first one, the second lies almost along the first axis (1 - |cos| of 1e-4 to
+    5e-4) and is preferred by its key so far that the third, at a right angle to it, wins or loses by little; the others are
+    far away.  Returns what the search takes, queries and keys without their other 15 components."""
+    H, cell = 8, 60.0
+    turn = np.linalg.qr(rng.normal(size=(B, 3, 3)))[0]
+    r = turn[:, :2] * rng.uniform(1.5, 2.5, (B, 2, 1))
+    far = np.stack([8.0 + 1.0 * np.arange(atoms - 3), 0 * np.arange(atoms - 3.0), 9.0 + 0 * np.arange(atoms - 3.0)], -1)
+    pos = (30.0 + np.concatenate([np.zeros((B, 1, 3)), r, np.broadcast_to(far, (B, atoms - 3, 3))], 1)).astype(np.float32)
+    rel = pos[:, 1:3].astype(np.float64) - pos[:, :1]
+    e1 = rel[:, 0] / np.linalg.norm(rel[:, 0], axis=-1, keepdims=True)
+    e2 = rel[:, 1] - (rel[:, 1] * e1).sum(-1, keepdims=True) * e1
+    e2 /= np.linalg.norm(e2, axis=-1, keepdims=True)
+    c1 = 1.0 - 10.0 ** rng.uniform(-4.0, -3.3, (B, H, 1))
+    f1 = np.zeros((B, atoms, H, 3))
+    f1[..., 0] = 1.0
+    f1[:, 0] = c1 * e1[:, None] + np.sqrt(length ** 2 - c1 ** 2) * np.cross(e1, e2)[:, None]
+    f1 = f1.astype(np.float32)
+    open1 = 1.0 - (rel[:, None, 0] * f1[:, 0]).sum(-1) / np.linalg.norm(rel[:, None, 0], axis=-1)
+    d2 = (rel ** 2).sum(-1)[:, None]
+    key = np.zeros((B, atoms, H))                                                                          # a = -1
+    key[:, 1] = d2[..., 0] - d2[..., 1] - np.log(np.maximum(open1, 1e-6)) - rng.uniform(-1e-3 * length, 3e-3 * length, (B, H))
+    t = lambda x: x.reshape((B * atoms,) + x.shape[2:]).astype(np.float32)
+    return t(pos), np.tile(np.eye(3, dtype=np.float32) * cell, (B, 1, 1)), t(np.ones((B, atoms, H))), t(key), t(f1)
+
+
+@pytest.mark.parametrize("atoms,crystals", [(3, 4000), (40, 400)])          # thread per pair, warp per atom and head
+@pytest.mark.parametrize("length", [1.0, 4.0, 30.0])
+def test_pruned_second_axis_selects_as_the_full_search(atoms, crystals, length):
+    """The second axis searched with lists, where pairs that cannot win are left out, selects the pair and image that it selects
+    without them, also behind images that are all but collinear with the first axis, and for first axes that are not of unit
+    length (a caller's own): 1 - |cos| is then a small difference of large numbers, and what a pair is said to reach has to
+    allow for its error."""
+    if not torch.cuda.is_available():
+        pytest.skip("no CUDA device")
+    from crystalframer_b200 import _lib
+    from crystalframer_b200.encoder import build_pair_list
+    dev = torch.device("cuda:0")
+    _configure()
+    made = _close_second_axis(crystals, atoms, length, np.random.default_rng(int(length) + atoms))
+    pos, cells, q, k, f1 = (torch.from_numpy(x).to(dev) for x in made)
+    edges, e_start, batch, _ = build_pair_list(torch.full((crystals,), atoms, dtype=torch.int64, device=dev))
+    pos_ij = (pos[edges[1]] - pos[edges[0]]).contiguous()
+    N, E, H = len(pos), edges.shape[1], 8
+    q, k = (torch.nn.functional.pad(x[..., None], (0, 15)).contiguous() for x in (q, k))
+    a = torch.full((N, H), -1.0, device=dev)
+    rvlen = torch.full((crystals, 3), 2 * np.pi / 60.0, device=dev)
+    p, ip = _lib.ptr, _lib.iptr
+    cache, lists = torch.empty(E, 4, device=dev), torch.empty(E, 5, 128, device=dev)
+    _lib.invoke("cfb200_pair_cache", 2, dev, p(pos_ij), p(cells), ip(batch), ip(edges), N, E, 2, p(cache), p(lists))
+    found = []
+    for geometry in ((p(cache), p(lists), 2), (None, None, 0)):
+        out = torch.empty(N, H, 3, device=dev)
+        pair, image = torch.empty(N, H, dtype=torch.int64, device=dev), torch.empty(N, H, dtype=torch.int32, device=dev)
+        _lib.invoke("cfb200_max_frame_cached", 1, dev, 2, p(q), p(k), p(a), p(pos_ij), p(cells), p(rvlen), ip(batch), ip(edges),
+                    ip(e_start), N, E, -3.5, 11, p(f1), p(out), ip(pair), p(image, torch.int32), *geometry)
+        found.append((pair, image, out))
+    first = found[1][0].view(crystals, atoms, H)[:, 0] - e_start[:-1].view(crystals, atoms)[:, :1]
+    assert int((first == 1).sum()) > crystals and int((first == 2).sum()) > crystals         # both win often
+    for x, y in zip(*found):
+        assert torch.equal(x, y), int((x != y).sum())
+
+
 @pytest.mark.parametrize("sizes", [(1,), (5, 2, 1, 1, 1), (1, 4, 4), (7, 9, 3)])        # 1, 32, 33 and 139 pairs
 @pytest.mark.parametrize("rng", [1, 2])
 @pytest.mark.parametrize("offset", [0, 1])
