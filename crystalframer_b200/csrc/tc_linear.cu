@@ -1,7 +1,7 @@
 // The dense layers on the 5th-generation tensor cores: tcgen05.mma (kind::f16, bf16 operands) with FP32 accumulation in
-// tensor memory.  Every operand is split exactly into three bf16 numbers, and six of the nine products are formed:
+// tensor memory.  Every operand is split into three bf16 numbers, and six of the nine products are formed:
 //
-//   x = x0 + x1 + x2 (8 significant bits each)
+//   x = x0 + x1 + x2 (8 significant bits each; exact for |x| above 2^-110, below which x2 falls under bf16's smallest number)
 //   A B^T  ~  A0 B0^T + (A0 B1^T + A1 B0^T + A1 B1^T + A0 B2^T + A2 B0^T)      (what is dropped is below 2^-24 of a product)
 //
 // at the price of three TF32 products, whose two parts lose two bits of an operand.
@@ -9,8 +9,16 @@
 // would collect an error of one sign per instruction.  The A0 B0 products therefore go in turns to three accumulators and
 // the small products to a fourth; the epilogue adds the four in FP32.  Distance from 64 bits, of the result's norm, for
 // normal operands and 128 / 512 terms: 6.6e-8 / 7.8e-8 (16e-8 where one block takes all 512); a chain of FP32 fused
-// multiply-adds 20e-8 / 21e-8 (41e-8), three TF32 products 16e-8 / 16e-8 (44e-8).  Operands of one sign, and ReLU outputs,
-// fare no worse (6.8e-8 against 16e-8, 5.4e-8 against 14e-8).
+// multiply-adds 20e-8 / 21e-8 (41e-8), three TF32 products 16e-8 / 16e-8 (44e-8).  Operands of one sign: 7.1e-8 / 6.9e-8
+// (22e-8) against 17e-8 / 9.5e-8 (35e-8); ReLU outputs 5.4e-8 / 6.7e-8 (11e-8) against 14e-8 / 15e-8 (29e-8).
+// What is cut off grows with the terms, where a chain's error grows with their root, and most for operands of one sign, of
+// which nothing averages out.  Longer contractions therefore go in runs: the A0 B0 products to two accumulators, which
+// together with the small ones are added in FP32, behind every run, to a sum in the third one's place (tc_drain).
+// Products of more than 512 terms in runs of eight slices, K = 2 048 / 32 768, 1 024 rows, operands of one sign: 17e-8 / 18e-8,
+// without runs 22e-8 / 773e-8, FP32 18e-8 / 70e-8; 18 / 220 us, without 17 / 198, FP32 36 / 515.  Weight gradients of splits
+// of more than 160 rows in runs of four slices, 4 000 / 10 700 / 131 072 atoms, operands of one sign: 8.4e-8 / 8.2e-8 / 8.8e-8,
+// without runs 10e-8 / 26e-8 / 651e-8, FP32 8.5e-8 / 10.9e-8 / 33e-8; of both 10e-8 / 11e-8 / 18e-8, without 11e-8 / 15e-8 /
+// 206e-8, FP32 22e-8 / 34e-8 / 118e-8.  Per launch of a layer's two, 2 661 atoms 12.7 us, without runs 11.9; 10 700 33.5 / 30.7.
 //
 // One CTA of eight warps and one owns a 128 x 64 output tile (or, over a cluster, a part of its contraction).  Per 32-wide slice
 // of the contraction index the eight warps bring both operands from global memory through registers (two register sets:
@@ -30,7 +38,7 @@
 // What bounds it: up to 2 700 rows a chain of latencies (launch, first loads, four slices, epilogue), beyond that the
 // instructions of the split (issue slots 48 % busy, tensor pipe 18 %).  Kernel time, [128] -> [512] and [512] -> [128],
 // against FP32 in gemm_kernel: 400 rows 7.5 / 8.9 against 7.1 / 8.6 us, 600 rows 7.6 / 9.0 against 10.3 / 11.9, 2 661 rows
-// 10.6 / 12.0 against 17.4 / 19.3, 10 700 rows 25 / 25 against 52 / 59; weight gradients of a layer of 10 700 atoms 64 against
+// 10.6 / 12.0 against 17.4 / 19.3, 10 700 rows 25 / 25 against 52 / 59; weight gradients of a layer of 10 700 atoms 67 against
 // 190.  Measured and left: 16 warps that bring and split, and a block barrier per slice with the instructions issued by one
 // of them (27 / 29 us); operands transposed on their way to shared memory (27 / 35 us in data gradients).
 //
@@ -53,15 +61,19 @@ constexpr int kTcABytes = kTcM * kTcKc * 2, kTcBBytes = kTcN * kTcKc * 2;       
 constexpr int kTcStageBytes = 3 * (kTcABytes + kTcBBytes);      // A0, A1, A2, B0, B1, B2
 constexpr int kTcStages = 3;
 constexpr int kTcSmemBytes = kTcStages * kTcStageBytes + 1024;  // and alignment slack
-constexpr int kTcAcc = 3;                    // accumulators of the large products; the small ones' follows them
+constexpr int kTcAcc = 3;                    // accumulators of the large products (two, and the sum so far, where there are
+                                             // several runs); the small ones' follows them
 constexpr int kTcCols = 256;                 // tensor-memory columns: four accumulators
 constexpr int kTcTileLd = kTcN / 4 + 1;      // float4 per row of the finished tile (conflict-free writes by rows)
 static_assert((kTcM * kTcTileLd + kTcThreads) * 16 <= kTcStages * kTcStageBytes, "the finished tile, and column sums, fit the stages");
+// Slices of a contraction that is taken in one run, and of a run (see above): in one run as long as that is no farther from 64
+// bits than the chain of FP32 additions in the kernels of the FP32 pipe.
+constexpr int kTcWholeGemm = 16, kTcRunGemm = 8, kTcWholeWgrad = 5, kTcRunWgrad = 4;
 constexpr uint32_t kTcSpinLimit = 1u << 22;
 
 __device__ __forceinline__ uint32_t smem_u32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
 
-// Two numbers into three bf16 each (packed: x low, y high); every step is exact.  A number that is not finite, or rounds to
+// Two numbers into three bf16 each (packed: x low, y high); every step is exact (see above).  A number that is not finite, or rounds to
 // infinity, leaves a part that is not a number.
 __device__ __forceinline__ void tc_split2(float x, float y, uint32_t (&part)[3])
 {
@@ -183,10 +195,12 @@ __device__ __forceinline__ void tc_stash1(const float4* v, uint8_t* o)
 // CTA-wide state of one tile computation: the shared-memory stages with their mbarriers
 struct TcCta {
     uint8_t* stage;
-    uint32_t full, empty, tmem;              // mbarriers per stage: written by all warps; read by its instructions
-    uint32_t slices_done;
+    uint32_t full, empty, drained, tmem;     // mbarriers per stage: written by all warps; read by its instructions; of a run:
+    uint32_t slices_done;                    // added to the sum so far
+    uint32_t runs_drained;
     bool failed;
 };
+constexpr int kTcBarriers = 2 * kTcStages + 1;
 
 __device__ __forceinline__ void tc_begin(TcCta& T, uint8_t* smem_raw, uint64_t* mbar_slots, uint32_t* tmem_slot)
 {
@@ -194,13 +208,15 @@ __device__ __forceinline__ void tc_begin(TcCta& T, uint8_t* smem_raw, uint64_t* 
     T.stage = smem_raw + (base - smem_u32(smem_raw));
     T.full = smem_u32(mbar_slots);
     T.empty = T.full + 8 * kTcStages;
-    T.slices_done = 0;
+    T.drained = T.empty + 8 * kTcStages;
+    T.slices_done = T.runs_drained = 0;
     T.failed = false;
     if (threadIdx.x == 0) {
         for (int i = 0; i < kTcStages; i++) {
             asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(T.full + 8 * i), "r"(kTcThreads / 32) : "memory");
             asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(T.empty + 8 * i) : "memory");
         }
+        asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(T.drained), "r"(kTcThreads / 32) : "memory");
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     if ((threadIdx.x >> 5) == 0) {
@@ -228,15 +244,22 @@ __device__ __forceinline__ void tc_slice(TcCta& T, const TcSlice& S)
     if ((threadIdx.x & 31) == 0) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(T.full + 8 * st) : "memory");
 }
 
-// One thread of the last warp: the instructions of `total` slices, each when its stage is full.
-template <bool TRA, bool TRB>
+// One thread of the last warp: the instructions of `total` slices, each when its stage is full, those of a run's first one
+// when the run before has been drained.  RUN: slices of a run; 0: one run takes all.
+template <bool TRA, bool TRB, int RUN>
 __device__ __forceinline__ void tc_issue(TcCta& T, const int total)
 {
     constexpr uint32_t idesc = tc_idesc<TRA, TRB>();
     constexpr uint64_t pa = kTcABytes >> 4, pb = kTcBBytes >> 4;      // from part to part, in descriptor units of 16 bytes
     const uint32_t small = T.tmem + kTcAcc * kTcN;
+    constexpr uint32_t accs = RUN > 0 ? kTcAcc - 1 : kTcAcc;
+    uint32_t in_run = 0, runs = 0;
     for (uint32_t s = 0; s < (uint32_t)total; s++) {
         const uint32_t round = s / kTcStages, st = s - round * kTcStages;
+        if (RUN > 0 && in_run == RUN) {
+            in_run = 0;
+            if (!tc_wait(T.drained, runs++ & 1)) T.failed = true;
+        }
         if (!tc_wait(T.full + 8 * st, round & 1)) T.failed = true;
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         const uint32_t base = smem_u32(T.stage) + st * kTcStageBytes;
@@ -244,14 +267,15 @@ __device__ __forceinline__ void tc_issue(TcCta& T, const int total)
 #pragma unroll
         for (uint32_t k = 0; k < kTcKc / 16; k++) {
             const uint64_t a = a0 + k * tc_kstep(TRA), b = b0 + k * tc_kstep(TRB);
-            const uint32_t n = s * (kTcKc / 16) + k;
-            tc_mma(T.tmem + (n % kTcAcc) * kTcN, a, b, idesc, n >= (uint32_t)kTcAcc ? 1u : 0u);
+            const uint32_t n = in_run * (kTcKc / 16) + k;
+            tc_mma(T.tmem + (n % accs) * kTcN, a, b, idesc, n >= accs ? 1u : 0u);
             tc_mma(small, a, b + pb, idesc, n > 0 ? 1u : 0u);
             tc_mma(small, a + pa, b, idesc, 1u);
             tc_mma(small, a + pa, b + pb, idesc, 1u);
             tc_mma(small, a, b + 2 * pb, idesc, 1u);
             tc_mma(small, a + 2 * pa, b, idesc, 1u);
         }
+        in_run++;
         asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(T.empty + 8 * st) : "memory");
     }
 }
@@ -267,20 +291,80 @@ __device__ __forceinline__ void tc_load16(uint32_t (&r)[16], uint32_t tmem, int 
         : "r"(addr) : "memory");
 }
 
+__device__ __forceinline__ void tc_load8(uint32_t (&r)[8], uint32_t addr)
+{
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];\n"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]) : "r"(addr) : "memory");
+}
+
+// waits for the loads; the loaded values must not be used, or moved, before that
+__device__ __forceinline__ void tc_loaded(uint32_t (&a)[8], uint32_t (&b)[8])
+{
+    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+    for (int i = 0; i < 8; i++) asm volatile("" : "+r"(a[i]), "+r"(b[i]));
+}
+
+// The eight warps that bring operands, once they have stored the second slice of the run behind it (the tensor core has done
+// with this one by then, and has two more slices to go on with): adds run `run` to the sum so far, which lies in the third
+// accumulator's place.  Rows and columns of a warp as in tc_finish.
+template <int RUN>
+__device__ __forceinline__ void tc_drain(TcCta& T)
+{
+    const uint32_t run = T.runs_drained++, s = (run + 1) * RUN - 1;
+    if (!tc_wait(T.empty + 8 * (s % kTcStages), (s / kTcStages) & 1)) T.failed = true;
+    __syncwarp();
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    const uint32_t base = T.tmem + ((uint32_t)(((threadIdx.x >> 5) & 3) * 32) << 16) + (threadIdx.x >> 7) * 32;
+#pragma unroll 1
+    for (uint32_t addr = base; addr < base + 32; addr += 8) {
+        uint32_t u[8], v[8], w[8];                              // (two at a time: the slices in flight take the registers)
+        tc_load8(u, addr);
+        tc_load8(v, addr + kTcN);
+        tc_loaded(u, v);
+#pragma unroll
+        for (int i = 0; i < 8; i++) u[i] = __float_as_uint(__uint_as_float(u[i]) + __uint_as_float(v[i]));
+        tc_load8(v, addr + kTcAcc * kTcN);
+        tc_load8(w, addr + 2 * kTcN);                           // the sum so far; in the first run of no meaning
+        tc_loaded(v, w);
+#pragma unroll
+        for (int i = 0; i < 8; i++) {
+            const float x = __uint_as_float(u[i]) + __uint_as_float(v[i]);
+            u[i] = __float_as_uint(run > 0 ? __uint_as_float(w[i]) + x : x);
+        }
+        asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};\n" ::"r"(addr + 2 * kTcN),
+                     "r"(u[0]), "r"(u[1]), "r"(u[2]), "r"(u[3]), "r"(u[4]), "r"(u[5]), "r"(u[6]), "r"(u[7]) : "memory");
+    }
+    asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    __syncwarp();
+    if ((threadIdx.x & 31) == 0) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(T.drained) : "memory");
+}
+
+// the run that is to be drained behind the slice just stored, if there is one
+template <int RUN>
+__device__ __forceinline__ void tc_drain_due(TcCta& T)
+{
+    if constexpr (RUN > 0)
+        if (T.slices_done == (T.runs_drained + 1) * RUN + 2) tc_drain<RUN>(T);
+}
+
 // Waits for the last slice (its commit covers every instruction issued before it), adds the accumulators and leaves the tile
 // in shared memory: row r at tile + r * kTcTileLd.  Returns it after a block barrier, tensor memory freed.  exact(m, n):
 // the element in plain FP32, for tiles with results that are not finite.
-template <class Exact>
+template <int RUN, class Exact>
 __device__ __forceinline__ float4* tc_finish(TcCta& T, const int total, Exact&& exact)
 {
     float4* tile = reinterpret_cast<float4*>(T.stage);
     const int row = ((threadIdx.x >> 5) & 3) * 32 + (threadIdx.x & 31), half = threadIdx.x >> 7;
+    const bool brings = threadIdx.x < kTcThreads;
+    if constexpr (RUN > 0)                                      // a last run of one slice has not drained the one before it
+        if (brings && (int)(T.runs_drained + 1) * RUN < total) tc_drain<RUN>(T);
     if (total > 0) {
         const uint32_t s = total - 1;
         if (!tc_wait(T.empty + 8 * (s % kTcStages), (s / kTcStages) & 1)) T.failed = true;
     }
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-    const bool brings = threadIdx.x < kTcThreads;
     __syncthreads();                                            // every warp knows that the stages are free
     float seen = 0.f;                                           // of this thread's outputs: finite when they are (or wrongly not)
     if (brings && total > 0) {
@@ -302,8 +386,9 @@ __device__ __forceinline__ float4* tc_finish(TcCta& T, const int total, Exact&& 
 #pragma unroll
                 for (int i = 0; i < 4; i++) {
                     const int x = 4 * q + i;
-                    // (a contraction of one slice of 32 has used two of the three accumulators)
-                    const float third = total > 1 ? __uint_as_float(u[2][x]) : 0.f;
+                    // (a contraction of one slice of 32 has used two of the three accumulators; behind several runs this is
+                    // the sum of all but the last)
+                    const float third = total > (RUN > 0 ? RUN : 1) ? __uint_as_float(u[2][x]) : 0.f;
                     v[i] = ((__uint_as_float(u[0][x]) + __uint_as_float(u[1][x])) + third) + __uint_as_float(u[3][x]);
                     seen += v[i];
                 }
@@ -329,11 +414,11 @@ __device__ __forceinline__ float4* tc_finish(TcCta& T, const int total, Exact&& 
 }
 
 // ---- C = sum_s A_s op(B_s) (+ bias) (+ residual), ReLU / mask: same contract as gemm_kernel (linear.cu) ----------
-template <bool B_KN>
+template <bool B_KN, int RUN>
 __global__ void __launch_bounds__(kTcBlock, 2) tc_gemm_kernel(const GemmBatch Gb)
 {
     extern __shared__ uint8_t tc_smem[];
-    __shared__ uint64_t mbar_slots[2 * kTcStages];
+    __shared__ uint64_t mbar_slots[kTcBarriers];
     __shared__ uint32_t tmem_slot;
     const GemmArgs& G = Gb.g[blockIdx.z / Gb.splits];
     const int rank = blockIdx.z % Gb.splits;
@@ -369,14 +454,14 @@ __global__ void __launch_bounds__(kTcBlock, 2) tc_gemm_kernel(const GemmBatch Gb
     if (brings) { fetch(R0); fetch(R1); }
     if (brings) {
         for (int s = 0; s < total; s += 2) {
-            tc_slice<false, B_KN>(T, R0); fetch(R0);
-            if (s + 1 < total) { tc_slice<false, B_KN>(T, R1); fetch(R1); }
+            tc_slice<false, B_KN>(T, R0); fetch(R0); tc_drain_due<RUN>(T);
+            if (s + 1 < total) { tc_slice<false, B_KN>(T, R1); fetch(R1); tc_drain_due<RUN>(T); }
         }
     } else if (threadIdx.x == kTcThreads) {
-        tc_issue<false, B_KN>(T, total);
+        tc_issue<false, B_KN, RUN>(T, total);
     }
     __syncwarp();
-    float4* tile = tc_finish(T, total, [&](const int r, const int c) {
+    float4* tile = tc_finish<RUN>(T, total, [&](const int r, const int c) {
         float v = 0.f;
         const int m = m0 + r, n = n0 + c;
         if (m >= G.M || n >= G.N) return v;
@@ -427,11 +512,18 @@ static bool tc_gemm_covers(const GemmBatch& Gb)
     return true;
 }
 
-template <bool B_KN>
+static int tc_slices(const GemmArgs& G)
+{
+    int slices = 0;
+    for (int s = 0; s < G.nseg; s++) slices += G.seg[s].K / kTcKc;
+    return slices;
+}
+
+template <bool B_KN, int RUN>
 static int launch_tc_gemm(GemmBatch& Gb, cudaStream_t st)
 {
     const GemmArgs& G = Gb.g[0];
-    auto kern = tc_gemm_kernel<B_KN>;
+    auto kern = tc_gemm_kernel<B_KN, RUN>;
     static std::atomic<bool> attr_done[64];
     int dev = 0;
     cudaGetDevice(&dev);
@@ -439,8 +531,7 @@ static int launch_tc_gemm(GemmBatch& Gb, cudaStream_t st)
         if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kTcSmemBytes) != cudaSuccess) return CFB200_E_CUDA;
         attr_done[dev & 63] = true;
     }
-    int slices = 0;
-    for (int s = 0; s < G.nseg; s++) slices += G.seg[s].K / kTcKc;
+    const int slices = tc_slices(G);
     const unsigned gx = (unsigned)((G.M + kTcM - 1) / kTcM), gy = (unsigned)(G.N / kTcN);
     // blocks that share a tile's contraction: as many as have four slices each, up to four, while all are resident at once
     int splits = slices / 4 < 4 ? slices / 4 : 4;
@@ -463,16 +554,20 @@ static int launch_tc_gemm(GemmBatch& Gb, cudaStream_t st)
 
 static int tc_gemm_batch(GemmBatch& Gb, bool b_kn, cudaStream_t st)
 {
-    return b_kn ? launch_tc_gemm<true>(Gb, st) : launch_tc_gemm<false>(Gb, st);
+    bool whole = true;
+    for (int i = 0; i < Gb.n; i++) whole = whole && tc_slices(Gb.g[i]) <= kTcWholeGemm;
+    if (whole) return b_kn ? launch_tc_gemm<true, 0>(Gb, st) : launch_tc_gemm<false, 0>(Gb, st);
+    return b_kn ? launch_tc_gemm<true, kTcRunGemm>(Gb, st) : launch_tc_gemm<false, kTcRunGemm>(Gb, st);
 }
 
 // ---- weight gradients: out[P,Q] = A[M,P]^T B[M,Q], rows split over gridDim.y, partial tiles to scratch -------
 // Same problem table, scratch layout and reduction as wgrad_kernel (linear.cu); tiles are 128 x 64 and both operands are
 // staged transposed (the contraction index, the atom, is the slow index of A and B in memory).
+template <int RUN>
 __global__ void __launch_bounds__(kTcBlock, 2) tc_wgrad_kernel(const WgArgs W)
 {
     extern __shared__ uint8_t tc_smem[];
-    __shared__ uint64_t mbar_slots[2 * kTcStages];
+    __shared__ uint64_t mbar_slots[kTcBarriers];
     __shared__ uint32_t tmem_slot;
     const int tid = threadIdx.x;
     int pi = 0;
@@ -505,14 +600,14 @@ __global__ void __launch_bounds__(kTcBlock, 2) tc_wgrad_kernel(const WgArgs W)
     tc_begin(T, tc_smem, mbar_slots, &tmem_slot);
     if (brings) {
         for (int s = 0; s < total; s += 2) {
-            step(R0); fetch(R0);
-            if (s + 1 < total) { step(R1); fetch(R1); }
+            step(R0); fetch(R0); tc_drain_due<RUN>(T);
+            if (s + 1 < total) { step(R1); fetch(R1); tc_drain_due<RUN>(T); }
         }
     } else if (tid == kTcThreads) {
-        tc_issue<true, true>(T, total);
+        tc_issue<true, true, RUN>(T, total);
     }
     __syncwarp();
-    const float4* tile = tc_finish(T, total, [&](const int p, const int q) {
+    const float4* tile = tc_finish<RUN>(T, total, [&](const int p, const int q) {
         float v = 0.f;
         for (int r = r0; r < r1; r++) v = fmaf(__ldg(Pb.A + (size_t)r * Pb.lda + p0 + p), __ldg(Pb.B + (size_t)r * Pb.ldb + q0 + q), v);
         return v;
@@ -542,17 +637,23 @@ static bool tc_wgrad_covers(const WgProblem& Pb, int64_t M)
     return M >= kTcMinRows && Pb.nb == 1 && Pb.P % kTcM == 0 && Pb.Q % kTcN == 0;
 }
 
-static int tc_wgrad_launch(const WgArgs& W, int tiles, cudaStream_t st)
+template <int RUN>
+static int launch_tc_wgrad(const WgArgs& W, int tiles, cudaStream_t st)
 {
     static std::atomic<bool> attr_done[64];
     int dev = 0;
     cudaGetDevice(&dev);
     if (!attr_done[dev & 63]) {
-        if (cudaFuncSetAttribute(tc_wgrad_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kTcSmemBytes) != cudaSuccess) return CFB200_E_CUDA;
+        if (cudaFuncSetAttribute(tc_wgrad_kernel<RUN>, cudaFuncAttributeMaxDynamicSharedMemorySize, kTcSmemBytes) != cudaSuccess) return CFB200_E_CUDA;
         attr_done[dev & 63] = true;
     }
-    tc_wgrad_kernel<<<dim3(tiles, W.S), kTcBlock, kTcSmemBytes, st>>>(W);
+    tc_wgrad_kernel<RUN><<<dim3(tiles, W.S), kTcBlock, kTcSmemBytes, st>>>(W);
     return cudaGetLastError() == cudaSuccess ? CFB200_OK : CFB200_E_CUDA;
+}
+
+static int tc_wgrad_launch(const WgArgs& W, int tiles, cudaStream_t st)
+{
+    return W.rows <= kTcWholeWgrad * kTcKc ? launch_tc_wgrad<0>(W, tiles, st) : launch_tc_wgrad<kTcRunWgrad>(W, tiles, st);
 }
 
 }  // namespace cfb

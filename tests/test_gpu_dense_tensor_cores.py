@@ -1,7 +1,7 @@
 """Dense layers on the tensor cores: around the row tile (128) and the smallest batch that takes them (512), contractions of
 one slice (32), of three and of those that two to four blocks share, one to three tiles of 64 outputs, both layouts of the
-weight -- against float64; operands that are not finite; weight and bias gradients, which only a layer has, against framework
-products."""
+weight -- against float64; contractions taken in several runs; operands that are not finite; weight and bias gradients, which
+only a layer has, against framework products, and the weights' against float64 up to 65 537 atoms."""
 import numpy as np
 import pytest
 import torch
@@ -47,6 +47,62 @@ def test_products(rows, outs, inner, kn):
     size += b.double().abs() + r.double().abs()
     assert ((y2.double() - want).abs() <= (inner / 16 + 7) * 2.0 ** -23 * size).all()
     assert torch.equal(y2, _linear(x, w, b, r, 1, kn))
+
+
+@pytest.mark.parametrize("rows,outs,inner", [(10000, 192, 512), (10000, 192, 544), (10000, 192, 576), (10000, 192, 768), (10000, 192, 1024),
+                                             (513, 64, 1056), (700, 128, 2080), (520, 64, 8192)])
+@pytest.mark.parametrize("kn", [0, 1])
+@pytest.mark.parametrize("signs", [1, 2])
+def test_products_of_long_contractions(rows, outs, inner, kn, signs):
+    """Contractions above 512 terms, which one block takes in runs of eight slices (last runs of one, of two and of eight), or
+    which blocks share: distance from float64, of the result's norm, for operands of both signs and of one.  The accumulators
+    cut off what does not fit, on average 2^-24 of their size: a run's eight times (16 where one takes 512 terms), while they
+    grow, so half of 8 (16) times that, and the runs' FP32 sum adds below 2^-24 per eighth of their number's root."""
+    x, w, _, _ = _draw(rows, outs, inner, kn)
+    if signs == 1:
+        x, w = x.abs(), w.abs()
+    y = _linear(x, w, None, None, 0, kn)
+    want = x.double() @ (w.double() if kn else w.double().t())
+    error = float((y.double() - want).norm() / want.norm())
+    assert error <= (4 if inner > 512 else 8) * 2.0 ** -24 * 1.25, error
+    x[5, 7], x[rows - 1, inner - 1] = float("inf"), float("nan")
+    z = _linear(x, w, None, None, 0, kn)
+    assert z[rows - 1].isnan().all() and not z[5].isfinite().any() and torch.equal(z[128:rows // 128 * 128], y[128:rows // 128 * 128])
+
+
+@pytest.mark.parametrize("atoms", [600, 2560, 2593, 3500, 4000, 4600, 16384, 65537])
+@pytest.mark.parametrize("signs", [1, 2])
+def test_weight_gradients_of_large_batches(atoms, signs):
+    """Feed-forward weight gradients of a layer against float64 on the activations that the layer's own products give: splits
+    of the atoms that one run takes (up to 160) and of two to 33 runs of four slices, last ones of one, two, three and four.
+    The accumulators of the large products are cut off four times by 2^-24 of their size on average, while they grow: 2 2^-24
+    at most for operands of one sign, less the first of each, which cuts nothing off; the FP32 sums of the runs and of the 16
+    splits add roundings of either sign, below 2^-24 in all.  Of both signs the result is smaller than its parts: twice that."""
+    if not torch.cuda.is_available():
+        pytest.skip("no CUDA device")
+    from crystalframer_b200 import _lib, data, synth
+    from crystalframer_b200.latticeformer import Latticeformer, ModelParams
+    dev = torch.device("cuda:0")
+    torch.manual_seed(1)
+    model = Latticeformer(ModelParams(num_layers=1, frame_method="no", value_pe_angle_real=0, symm_break_noise=0.0)).to(dev).train()
+    layer = model.encoder.layers[0]
+    with torch.no_grad():
+        model(data.host_batch(synth.make_batch(16, 3), np.zeros((16, 1), np.float32), pinned=False).to(dev, non_blocking=False))
+        layer.self_attn.out_proj.weight.zero_()                 # the feed-forward block's input is the layer's
+    g = torch.Generator().manual_seed(atoms)
+    x, up = (torch.randn(atoms, 128, generator=g).to(dev) for _ in range(2))
+    if signs == 1:
+        x, up = x.abs(), up.abs()
+    eye = torch.eye(3, device=dev).expand(atoms, 3, 3).contiguous()
+    one = torch.arange(atoms, device=dev)
+    model.zero_grad(set_to_none=True)
+    layer(x, one, one.repeat(2, 1), torch.zeros(atoms, 3, device=dev), None, 6 * eye, None, eye, None).backward(up)
+    w1, b1, w2 = (p.detach() for p in (layer.linear1.weight, layer.linear1.bias, layer.linear2.weight))
+    h = _linear(x, w1, b1, None, 1, 0)
+    gh = torch.where(h > 0, _linear(up, w2, None, None, 0, 1), 0.0)
+    for got, want in ((layer.linear2.weight.grad, up.double().t() @ h.double()), (layer.linear1.weight.grad, gh.double().t() @ x.double())):
+        error = float((got.double() - want).norm() / want.norm())
+        assert error <= 2.5 * signs * 2.0 ** -24, error
 
 
 @pytest.mark.parametrize("kn", [0, 1])
