@@ -1417,13 +1417,17 @@ __global__ void __launch_bounds__(kOrWarps * 32, 2) attn_ordered_kernel(const __
 // Backward pass from the results of the training forward.  Per pair
 //   p = exp(q.k + z - lse),  gz = p (gout . (v_j + values_ij) - gout . out_i),
 //   ga += c_dist x gz - p x gout . values_ij,  gq += gz k_j;   and ga += gout . upool once per atom
-// (the coefficient gradient as in the recomputing backward, reference quirk included).  Block = (atom, eight heads), lane =
+// (the coefficient gradient as in the recomputing backward, reference quirk included).  Block = (atom, up to eight heads), lane =
 // (head, four of the 16 components), so that a row of keys, values or value encodings is one contiguous 512-byte read: a lane
 // that took a whole head's 64 bytes would touch a cache line per lane and load, and the tags of the L1 cache set the pace (12
 // LDG.128 x 32 lines for 32 pairs of a head).  The dot products meet over four lanes.  Eight warps share the atom's pairs, one
 // pair at a time each: latency is covered by warps (64 registers, 32 warps per SM), which does better than two or four pairs in
 // flight per warp.  Bound by the latency of the reads.  Per launch, 256 log-normal crystals 49 -> 27 us (two pairs in flight 38),
 // 16 cells of 100-200 atoms 145 -> 72 us (111).
+// HB: heads side by side; with fewer than eight the rest of a warp takes other pairs of the atom, WA warps an atom, and a block
+// 8 / WA atoms: 16 pairs of an atom in flight.  With the column pass behind it, a warp per (atom, head) and lane = pair / eight
+// lanes groups of which those beyond the last head idle / this: one head, 256 log-normal crystals 12.6 / 18.3 / 11.9 us, 1 024
+// 33 / 58 / 29, 16 cells of 100-200 atoms 22.5 / 44 / 18.8; two heads, 1 024 crystals 72 / 76 / 54; four 113 / 93 / 91.
 constexpr int kBsWarps = 8;
 
 __device__ __forceinline__ float quad_sum(float v)
@@ -1434,13 +1438,17 @@ __device__ __forceinline__ float quad_sum(float v)
 
 __device__ __forceinline__ float dot4(const float4 a, const float4 b) { return fmaf(a.x, b.x, fmaf(a.y, b.y, fmaf(a.z, b.z, a.w * b.w))); }
 
+template <int HB, int WA>
 __global__ void __launch_bounds__(kBsWarps * 32) attn_bwd_saved_kernel(const AtArgs A, const Params P)
 {
     wait_for_predecessors();
+    constexpr int kAtoms = kBsWarps / WA, kSub = 8 / HB;    // atoms of a block, WA warps each; pairs side by side in a warp
+    constexpr int kSlots = WA * kSub;                       // pairs of an atom in flight
     const int H = P.H, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int64_t i = blockIdx.x;
-    const int head = blockIdx.y * 8 + (lane >> 2), h = min(head, H - 1);       // lanes beyond the last head repeat it
-    const bool live = head < H;
+    const int64_t ia = (int64_t)blockIdx.x * kAtoms + warp / WA;
+    const int64_t i = kAtoms == 1 ? ia : min(ia, A.N - 1);                         // warps beyond the last atom repeat it
+    const int h = blockIdx.y * HB + (lane >> 2) % HB;
+    const bool live = kAtoms == 1 || ia < A.N;
     const int64_t ih = i * H + h;
     const int c0 = (lane & 3) * 4;
     auto load4 = [&](const float* src, const int64_t row) { return __ldg(reinterpret_cast<const float4*>(src + row * kAtHd + c0)); };
@@ -1452,35 +1460,54 @@ __global__ void __launch_bounds__(kBsWarps * 32) attn_bwd_saved_kernel(const AtA
     float4 gq = make_float4(0.f, 0.f, 0.f, 0.f);
     float ga = 0.f;
 #pragma unroll 1
-    for (int64_t e = e0 + warp; e < e1; e += kBsWarps) {
-        const int64_t j = j0 + (e - e0);
+    for (int64_t e_w = e0 + warp % WA * kSub; e_w < e1; e_w += kSlots) {
+        const bool on = kSub == 1 || e_w + (lane >> 2) / HB < e1;
+        const int64_t e = kSub == 1 ? e_w : min(e_w + (lane >> 2) / HB, e1 - 1), j = j0 + (e - e0);
         const float4 k = load4(A.k, j * H + h), v = load4(A.v, j * H + h), x = load4(A.val, e * H + h);
         const float z = __ldg(A.z_in + e * H + h), px = __ldg(A.px + e * H + h);
         const float qk = quad_sum(dot4(q, k)), gov = quad_sum(dot4(g, v)), cB = quad_sum(dot4(g, x));
         const float p = __expf(qk + z - lse);
         const float gz = p * (gov + cB - D);
-        if (live && (lane & 3) == 0) A.gz[e * H + h] = gz;
-        ga += px * fmaf(P.c_dist, gz, -p * cB);
-        gq.x = fmaf(gz, k.x, gq.x); gq.y = fmaf(gz, k.y, gq.y); gq.z = fmaf(gz, k.z, gq.z); gq.w = fmaf(gz, k.w, gq.w);
+        if (on) {
+            if (live && (lane & 3) == 0) A.gz[e * H + h] = gz;
+            ga += px * fmaf(P.c_dist, gz, -p * cB);
+            gq.x = fmaf(gz, k.x, gq.x); gq.y = fmaf(gz, k.y, gq.y); gq.z = fmaf(gz, k.z, gq.z); gq.w = fmaf(gz, k.w, gq.w);
+        }
     }
-    // the warps' parts, in a fixed order
+    // an atom's parts, by its pairs modulo the slots, in a fixed order; the first warp takes all atoms and heads of the block
     __shared__ float part[kBsWarps][5][32];
     part[warp][0][lane] = gq.x; part[warp][1][lane] = gq.y; part[warp][2][lane] = gq.z; part[warp][3][lane] = gq.w;
     part[warp][4][lane] = ga;
     __syncthreads();
     if (warp > 0) return;
+    const int atom = lane / (4 * HB);                       // (its head is this lane's own)
+    const int64_t io = kAtoms == 1 ? i : (int64_t)blockIdx.x * kAtoms + atom;
+    if (atom >= kAtoms || io >= A.N) return;
+    auto at = [&](const int c, const int s) { return part[atom * WA + s / kSub][c][s % kSub * 4 * HB + lane % (4 * HB)]; };
     float r[5];
 #pragma unroll
     for (int c = 0; c < 5; c++) {
-        static_assert(kBsWarps == 8, "");
-        r[c] = ((part[0][c][lane] + part[1][c][lane]) + (part[2][c][lane] + part[3][c][lane])) +
-               ((part[4][c][lane] + part[5][c][lane]) + (part[6][c][lane] + part[7][c][lane]));
+        static_assert(kSlots == 8 || kSlots == 16, "");
+        r[c] = ((at(c, 0) + at(c, 1)) + (at(c, 2) + at(c, 3))) + ((at(c, 4) + at(c, 5)) + (at(c, 6) + at(c, 7)));
+        if (kSlots == 16)
+            r[c] += ((at(c, 8) + at(c, 9)) + (at(c, 10) + at(c, 11))) + ((at(c, 12) + at(c, 13)) + (at(c, 14) + at(c, 15)));
     }
-    const float gup = quad_sum(dot4(g, load4(A.upool, ih)));
-    if (live) {
-        *reinterpret_cast<float4*>(A.gq + ih * kAtHd + c0) = make_float4(r[0], r[1], r[2], r[3]);
-        if ((lane & 3) == 0) A.ga[ih] = r[4] + gup;
-    }
+    const int64_t oh = io * H + h;
+    const float4 go = kAtoms == 1 ? g : load4(A.gout, oh), up = load4(A.upool, oh);
+    const unsigned quad = 0xfu << (lane & ~3);
+    float gup = dot4(go, up);
+    gup += __shfl_xor_sync(quad, gup, 1);
+    gup += __shfl_xor_sync(quad, gup, 2);
+    *reinterpret_cast<float4*>(A.gq + oh * kAtHd + c0) = make_float4(r[0], r[1], r[2], r[3]);
+    if ((lane & 3) == 0) A.ga[oh] = r[4] + gup;
+}
+
+template <int HB, int WA>
+static void launch_bwd_saved(const AtArgs& A, const Params& P, cudaStream_t st)
+{
+    constexpr int atoms = kBsWarps / WA;
+    launch_ahead(attn_bwd_saved_kernel<HB, WA>, dim3((unsigned)((A.N + atoms - 1) / atoms), (unsigned)(P.H / HB)), kBsWarps * 32, 0, st,
+                 A, P);
 }
 
 // blocks per head: the resident ones of the device, no more than the head's atoms can feed
@@ -1707,7 +1734,10 @@ int attn_fused_bwd(const AtArgs& A, const Params& P, cudaStream_t st)
     if (A.N == 0) return CFB200_OK;
     if (A.val == nullptr) return launch_tile<2>(A, P, st);
     if (!on_grid({A.qs, A.k, A.v, A.gout, A.out, A.upool, A.val, A.gq})) return CFB200_E_SHAPE;
-    launch_ahead(attn_bwd_saved_kernel, dim3((unsigned)A.N, (unsigned)((P.H + 7) / 8)), kBsWarps * 32, 0, st, A, P);
+    if (P.H % 8 == 0) launch_bwd_saved<8, 8>(A, P, st);             // (the heads are a power of two)
+    else if (P.H == 4) launch_bwd_saved<4, 8>(A, P, st);
+    else if (P.H == 2) launch_bwd_saved<2, 4>(A, P, st);
+    else launch_bwd_saved<1, 2>(A, P, st);
     return cudaGetLastError() == cudaSuccess ? CFB200_OK : CFB200_E_CUDA;
 }
 
