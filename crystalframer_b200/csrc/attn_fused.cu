@@ -106,7 +106,7 @@ __host__ __device__ constexpr int fw_blocks(int mode) { return mode == 2 ? 4 : 2
 __host__ __device__ constexpr size_t fw_smem_bytes(int AH, int mode)
 {
     return sizeof(float) * (kAtHd * fw_k(AH) + fw_warps(mode) * (32 * kFwRec + 5 * kFwStage + fw_rows(mode) * fw_k(AH) +
-                                                                      (mode == 2 ? 2 * kFwWait * kFwWaitLd : 0)));
+                                                                      (mode == 2 && AH > 0 ? 2 * kFwWait * kFwWaitLd : 0)));
 }
 // translations whose weight is below exp(-24) = 4e-11 of the nearest one's do not enter the normaliser: the 125 of a
 // box together stay below a tenth of its last bit
@@ -452,8 +452,10 @@ __global__ void __launch_bounds__(fw_warps(MODE) * 32, fw_blocks(MODE)) attn_til
         if constexpr (MODE == 0) pooled([](const int, const float) { return 0.f; });
 
         // Backward: a pair's two sums over the lanes.  A butterfly per pair is seven dependent shuffles; eight pairs at once
-        // (lane = pair, quarter of the lanes) are 30 instructions, and the sums go to the lanes that hold the pairs.  64 cells
-        // of 100-200 atoms, backward with frames 1.92 -> 1.88 ms, without 1.36 -> 1.29.
+        // (lane = pair, quarter of the lanes) are 30 instructions, and the sums go to the lanes that hold the pairs.  Backward
+        // with the column pass, butterflies / eight at once: with frames 64 cells of 100-200 atoms 2.11 / 2.07 ms, 256
+        // log-normal crystals 0.51 / 0.51; but without frames 1.505 / 1.499, and in small cells, where nothing covers the wait
+        // for the other pairs, 256 crystals 0.262 / 0.300, 1 024 0.768 / 0.842: there each pair has its butterfly.
         int waiting_pairs = 0, slot = -1;
         auto drain = [&]() {
             __syncwarp();
@@ -472,6 +474,17 @@ __global__ void __launch_bounds__(fw_warps(MODE) * 32, fw_blocks(MODE)) attn_til
         // the tile's pair j is complete: into the pooled sums, and into the row that waits for its projection
         auto flush = [&](const int j) {
             if constexpr (BACK) {
+                if constexpr (AH == 0) {
+                    // both sums over the lanes at once: the lower half of the warp takes B, the upper A
+                    const bool up = lane & 16;
+                    float r = (up ? accA : accB) + __shfl_xor_sync(0xffffffffu, up ? accB : accA, 16);
+#pragma unroll
+                    for (int o = 8; o > 0; o >>= 1) r += __shfl_xor_sync(0xffffffffu, r, o);
+                    const float b = __shfl_sync(0xffffffffu, r, 0), c2 = __shfl_sync(0xffffffffu, r, 16);
+                    if (lane == j) { cB = b; cA = c2; }
+                    accA = accB = 0.f;
+                    return;
+                }
                 // the lanes' parts wait in shared memory until eight pairs are complete
                 wait[waiting_pairs * kFwWaitLd + lane] = make_float2(accB, accA);
                 if (lane == j) slot = waiting_pairs;
