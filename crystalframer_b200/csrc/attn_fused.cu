@@ -460,9 +460,11 @@ __global__ void __launch_bounds__(fw_warps(MODE) * 32, fw_blocks(MODE)) attn_til
         auto drain = [&]() {
             __syncwarp();
             const float2* p = wait + (lane & 7) * kFwWaitLd + (lane >> 3) * 8;
-            float b = 0.f, c2 = 0.f;
+            float2 x[8];
 #pragma unroll
-            for (int k = 0; k < 8; k++) { const float2 u = p[k]; b += u.x; c2 += u.y; }
+            for (int k = 0; k < 8; k++) x[k] = p[k];
+            float b = ((x[0].x + x[1].x) + (x[2].x + x[3].x)) + ((x[4].x + x[5].x) + (x[6].x + x[7].x));
+            float c2 = ((x[0].y + x[1].y) + (x[2].y + x[3].y)) + ((x[4].y + x[5].y) + (x[6].y + x[7].y));
             b += __shfl_xor_sync(0xffffffffu, b, 8); c2 += __shfl_xor_sync(0xffffffffu, c2, 8);
             b += __shfl_xor_sync(0xffffffffu, b, 16); c2 += __shfl_xor_sync(0xffffffffu, c2, 16);
             b = __shfl_sync(0xffffffffu, b, slot & 7); c2 = __shfl_sync(0xffffffffu, c2, slot & 7);
