@@ -864,23 +864,23 @@ __global__ void __launch_bounds__(fw_warps(MODE) * 32, fw_blocks(MODE)) attn_til
 
 // ---- the forward one pair after the other -------------------------------------------------------------------------
 // Warp = (atom, head), its pairs in order, lane = basis index throughout (LatticeLane), each pair's 16 x 256 projection by
-// itself, an online soft-max over the pairs; leaves per-pair results.  Same results as attn_tile_kernel to rounding.  Bound by
-// instruction issue: 800 per (pair, head) in cells of 100-200 atoms, nearly all of them fixed.  Two uses:
+// itself, an online soft-max over the pairs; leaves per-pair results; sweeps each pair's translations.  Same results as
+// attn_tile_kernel to rounding.  Bound by instruction issue.  Two uses:
 // * batches without translation lists, where the tiles are no faster (see attn_fused_fwd);
-// * the training forward of models with weighted-PCA frames, for its rounding: attn_ordered_kernel forms the same sums in
-//   tiles, and takes this way where a task's range has no list (a training step of 16 crystals of 100-200 atoms 16.8 ms with
-//   this kernel, 12.4 with that one, 8.2 with attn_tile_kernel).  An eigenvector of the second moments has a sign and, where eigenvalues are
-//   close, a direction that a last bit decides, and the ReLUs behind it turn with it.  In a batch whose errors have balanced
-//   signs the mean gradient is small, and one turned ReLU is then a quarter of its root mean square: of 150 batches of 16
-//   such crystals two moved by more than a tenth when the tiles' order of summation took the place of this one, while the
-//   frames of the first layer, which come before it, stayed equal to the bit.  Here the order is part of the result.
+// * tasks without a list in the training forward of models with weighted-PCA frames, whose order of summation is this one for
+//   its rounding (attn_ordered_kernel forms the same sums in tiles from the lists; a training step of 16 crystals of 100-200
+//   atoms 16.8 ms one pair after the other, 12.4 with that kernel, 8.2 with attn_tile_kernel).  An eigenvector of the second
+//   moments has a sign and, where eigenvalues are close, a direction that a last bit decides, and the ReLUs behind it turn with
+//   it.  In a batch whose errors have balanced signs the mean gradient is small, and one turned ReLU is then a quarter of its
+//   root mean square: of 150 batches of 16 such crystals two moved by more than a tenth when the tiles' order of summation took
+//   the place of this one, while the frames of the first layer, which come before it, stayed equal to the bit.  There the order
+//   is part of the result.
 constexpr int kPwStride = 260;         // W [16][260]: conflict-free 128-bit reads by 16 rows
 
 // per-(atom, head) inputs
 struct AtomTask {
     int64_t i, c, e0, e1;
     int R1, R2, R3;
-    bool use_list;
 };
 
 template <bool ANG>
@@ -902,21 +902,7 @@ __device__ __forceinline__ AtomTask load_atom(const AtArgs& A, const Params& P, 
     int Rl = 0;
     if (lane < 3) Rl = lattice_range_1d(P, L.a, P.cutoff_radius != 0.0f ? __ldg(A.rvlen + 3 * T.c + lane) : 0.0f);
     T.R1 = __shfl_sync(0xffffffffu, Rl, 0); T.R2 = __shfl_sync(0xffffffffu, Rl, 1); T.R3 = __shfl_sync(0xffffffffu, Rl, 2);
-    T.use_list = A.list != nullptr && T.R1 == A.cache_range && T.R2 == A.cache_range && T.R3 == A.cache_range;
     return T;
-}
-
-template <bool ANG>
-__device__ __forceinline__ void run_pair(const AtArgs& A, const Params& P, LatticeLane<2, ANG>& L, const AtomTask& T,
-                                         const int64_t e)
-{
-    L.reset();
-    if (T.use_list) {
-        L.run_list(P, A.list + (size_t)e * kListStride);
-    } else {
-        L.run_slabs(P, T.R1, T.R2, T.R3, __ldg(A.pos_ij + 3 * e), __ldg(A.pos_ij + 3 * e + 1), __ldg(A.pos_ij + 3 * e + 2),
-                    A.tvecs + 9 * T.c);
-    }
 }
 
 constexpr int kPwWarps = 12;
@@ -966,7 +952,9 @@ __device__ __forceinline__ void pairwise_task(const AtArgs& A, const Params& P, 
         if (lane == 0 && __ldg(A.edges + A.E + e) != j) atomicOr(&g_status, CFB200_ST_PAIR_LAYOUT);   // not the dense layout
         float kd = 0.f, vd = 0.f;
         if (lane < kAtHd) { kd = __ldg(A.k + (j * H + h) * kAtHd + lane); vd = __ldg(A.v + (j * H + h) * kAtHd + lane); }
-        run_pair(A, P, L, T, e);
+        L.reset();
+        L.run_slabs(P, T.R1, T.R2, T.R3, __ldg(A.pos_ij + 3 * e), __ldg(A.pos_ij + 3 * e + 1), __ldg(A.pos_ij + 3 * e + 2),
+                    A.tvecs + 9 * T.c);
         float r0 = L.sum_l, r1 = L.px_l, r2 = qd * kd;
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) {
@@ -1536,6 +1524,7 @@ static int at_grid_x(int64_t N, int H, int mode)
     return (int)want;
 }
 
+// blocks per head of the kernels that take pairs one after the other, and of attn_ordered_kernel
 static int pairwise_grid_x(int64_t N, int H)
 {
     int64_t want = (int64_t)sm_count() * 2 / H;
@@ -1543,6 +1532,16 @@ static int pairwise_grid_x(int64_t N, int H)
     const int64_t need = (N + 7) / 8;
     if (need < want) want = need < 1 ? 1 : need;
     return (int)want;
+}
+
+// Workers per head that the queue of a weighted-PCA training batch is cut for.  An atom's chunks are summed apart, so where the
+// cuts are is part of the result: this goes by the device and the batch alone, whatever shape the forward is launched in (it
+// was the number of warps of the first kernel that walked such a queue).
+static int ordered_plan_workers(int64_t N, int H)
+{
+    int64_t blocks = (int64_t)sm_count() * 2 / H;
+    if (blocks > (N + 7) / 8) blocks = (N + 7) / 8;
+    return (int)(blocks < 1 ? 1 : blocks) * 12;
 }
 
 // thread = (queue entry, head): the task table.  Entry (x, y, z, w) = atom, result row (the atom, or N + partial row of

@@ -164,7 +164,7 @@ constexpr int kListStride = kListLen * kListPlanes;
 constexpr float kAtPairCost = 350.0f, kAtTermCost = 70.0f;
 // Long tasks are cut into chunks of consecutive pairs whose partial results a small kernel merges afterwards
 // (see atom_order_kernel and attn_fused.cu): at most kSplitMaxChunks chunks of at least kSplitMinPairs pairs,
-// kSplitSlots partial rows per head, no task below kSplitMinTarget (attn_pairwise_kernel's: kSplitMinTargetPairwise)
+// kSplitSlots partial rows per head, no task below kSplitMinTarget (weighted-PCA training: kSplitMinTargetPairwise)
 // instructions is cut.  kSplitWideSphere: volume of
 // the pruning sphere (radius^2 = 16 / |a|) of a Gaussian two standard deviations wider than typical (|a| = 0.051).
 constexpr int kSplitSlots = CFB200_SPLIT_SLOTS, kSplitMaxChunks = 8, kSplitMinPairs = 4;

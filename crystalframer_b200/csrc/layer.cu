@@ -431,9 +431,10 @@ static int batch_geometry(const float* pos, const float* tvecs, const int64_t* s
     cfb::launch_ahead(cfb::cell_kernel, (unsigned)((B + 127) / 128), 128, 0, st,
                       tvecs, sizes, B, rvecs, rvlen, vcell, key, inv_vol);
     if (E > 0) cfb::launch_ahead(cfb::pos_ij_kernel, (unsigned)((E + 255) / 256), 256, 0, st, pos, edges, E, pos_ij);
-    // warps that serve one head's queue in the training forward, the launch the chunks are cut for
+    // warps that serve one head's queue in the training forward, the launch the chunks are cut for (weighted-PCA models: see
+    // ordered_plan_workers)
     const int heads = split != nullptr ? g_cfg.num_heads : 1;
-    const int workers = pairwise ? cfb::pairwise_grid_x(N, heads) * cfb::kPwWarps : cfb::at_grid_x(N, heads, 1) * cfb::fw_warps(1);
+    const int workers = pairwise ? cfb::ordered_plan_workers(N, heads) : cfb::at_grid_x(N, heads, 1) * cfb::fw_warps(1);
     cfb::launch_ahead(cfb::atom_order_kernel, 1, 1024, 0, st,
                       key, inv_vol, sizes, crystal_start, B, N, workers, pairwise ? 0.5f : 0.25f,
                       pairwise ? cfb::kSplitMinTargetPairwise : cfb::kSplitMinTarget, by_rank, start_of, want_of, slot_of, order, split);
@@ -541,7 +542,7 @@ int cfb200_encoder_layer_fwd(const cfb200_layer_desc* L, const cfb200_layer_weig
     rc = make_params(L->dist_max, L->cutoff_radius, P, !ang);
     if (rc != CFB200_OK) return rc;
     cudaStream_t st = S(stream);
-    // training with weighted-PCA frames: every sum of the forward in the order of attn_pairwise_kernel's comment
+    // training with weighted-PCA frames: every sum of the forward in the order that attn_pairwise_kernel's comment gives
     const bool pairwise = L->frame_method == 2 && St->val != nullptr;
 
     // input projections: q, k, v = x W^T + b, one launch

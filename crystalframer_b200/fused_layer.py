@@ -80,7 +80,7 @@ class LayerGeometry:
     @classmethod
     def from_raw(cls, pos, trans, sizes, N, E, cutoff, pairwise=False):
         """One call of cfb200_batch_geometry on raw positions (N,3), lattice vectors (B,3,3), sizes (B).  ``pairwise``: the
-        work queue is cut for the training forward of weighted-PCA models (attn_pairwise_kernel)."""
+        work queue is cut for the training forward of weighted-PCA models (attn_ordered_kernel)."""
         from .cuda_funcs.common import allocate_pair_list
         from .cuda_funcs.kernel_manager import KernelManager
         g = cls()
