@@ -638,36 +638,108 @@ def test_translation_lists_are_sorted(sizes, rng, offset):
     assert ((d2.double() - xyz.square().sum(-1)).abs() <= 3 * 2.0 ** -24 * xyz.square().sum(-1)).all()
 
 
-@pytest.mark.parametrize("method", ["max", "no", "weighted_pca"])
-def test_prediction_in_a_captured_graph(method):
-    """Kernels launched ahead of their predecessors' end keep their order in a captured graph: replays give the eager
-    prediction bit for bit, also on inputs that a kernel wrote just before."""
-    if not torch.cuda.is_available():
-        pytest.skip("no CUDA device")
+def _model_and_two_batches(method, crystals, lo, hi):
+    """A model of two layers that has measured its coefficient statistics, a batch, and other positions for it."""
     from crystalframer_b200 import data, synth
     from crystalframer_b200.latticeformer import Latticeformer, ModelParams
     dev = torch.device("cuda:0")
+    np.random.seed(0)                                       # the frames' noise, also of the measuring forward below
     torch.manual_seed(0)
     model = Latticeformer(ModelParams(num_layers=2, frame_method=method, value_pe_angle_real=0 if method == "no" else 64)).to(dev).train()
-    tb = data.host_batch(synth.make_batch(48, 5), np.zeros((48, 1), np.float32), pinned=False).to(dev, non_blocking=False)
+    put = lambda b: data.host_batch(b, np.zeros((len(b.sizes), 1), np.float32), pinned=False).to(dev, non_blocking=False)
+    b = synth.make_batch(crystals, 5, size_dist="uniform", size_lo=lo, size_hi=hi, len_lo=3.0 + lo / 8, len_hi=9.0 + lo / 4)
+    tb = put(b)
     with torch.no_grad():
-        model(tb)
+        model(put(synth.make_batch(48, 5)))
+    g = torch.Generator().manual_seed(9)
+    moved = tb.pos + 0.3 * torch.randn(tb.pos.shape, generator=g).to(dev)
+    return model, tb, (tb.pos.clone(), moved)
+
+
+def _seeded(f):
+    np.random.seed(3)
+    torch.manual_seed(3)
+    return f()
+
+
+def _replays_follow(tb, sets, wanted, graph, got):
+    """Replays of a captured graph on either set of positions, which a kernel writes just before, into buffers that held no
+    numbers, give what was wanted of it bit for bit."""
+    for n in (1, 0, 1):
+        for x in got:
+            x.fill_(float("nan"))
+        tb.pos.copy_(sets[n])
+        graph.replay()
+        torch.cuda.synchronize()
+        for x, y in zip(got, wanted[n]):
+            assert torch.equal(x, y)
+
+
+BATCH_SHAPES = [("max", 96, 1, 20), ("max", 12, 40, 60), ("no", 96, 1, 20), ("no", 12, 40, 60), ("weighted_pca", 12, 40, 60)]
+
+
+@pytest.mark.parametrize("method,crystals,lo,hi", BATCH_SHAPES)
+def test_prediction_in_a_captured_graph(method, crystals, lo, hi):
+    """Kernels launched ahead of their predecessors' end keep their order in a captured graph: replays give the eager
+    predictions for two sets of positions in turn, each written by a kernel just before the replay."""
+    if not torch.cuda.is_available():
+        pytest.skip("no CUDA device")
+    from crystalframer_b200.cuda_funcs import common
+    model, tb, sets = _model_and_two_batches(method, crystals, lo, hi)
     model.eval()
 
     def predict():
-        np.random.seed(3)
-        torch.manual_seed(3)
         with torch.no_grad():
-            return model(tb)
-    side = torch.cuda.Stream()
-    with torch.cuda.stream(side):
-        want = predict()
-    side.synchronize()
+            return [model(tb)]
+    wanted = []
+    for pos in sets:
+        tb.pos.copy_(pos)
+        wanted.append(_seeded(predict))
+    assert not torch.equal(wanted[0][0], wanted[1][0])
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    common._FREE_MEMORY.clear()                             # the free memory is asked for in the capture too
+    with torch.cuda.graph(graph):
+        got = _seeded(predict)
+    _replays_follow(tb, sets, wanted, graph, got)
+
+
+def _gradients(model, tb):
+    params = [p for p in model.parameters() if p.requires_grad]
+    out = model(tb)
+    return [out.detach(), *[g for g in torch.autograd.grad(out.square().sum(), params, allow_unused=True) if g is not None]]
+
+
+def _write_serial_gradients(path, *shape):
+    model, tb, sets = _model_and_two_batches(*shape)
+    wanted = []
+    for pos in sets:
+        tb.pos.copy_(pos)
+        wanted.append([x.cpu() for x in _seeded(lambda: _gradients(model, tb))])
+    torch.save(wanted, path)
+
+
+@pytest.mark.parametrize("method,crystals,lo,hi", BATCH_SHAPES)
+def test_training_step_in_a_captured_graph(method, crystals, lo, hi, tmp_path):
+    """Forward and backward, weight gradients on their side stream, captured and replayed on two sets of positions in turn: every
+    gradient bit for bit that of a process that keeps all kernels on one stream, without a graph; eagerly too."""
+    if not torch.cuda.is_available():
+        pytest.skip("no CUDA device")
+    import os
+    import subprocess
+    import sys
+    here, path = os.path.dirname(os.path.abspath(__file__)), str(tmp_path / "wanted.pt")
+    subprocess.run([sys.executable, "-c", f"import sys; sys.path[:0] = [{os.path.dirname(here)!r}, {here!r}]; import test_gpu_properties as t; "
+                    f"t._write_serial_gradients({path!r}, {method!r}, {crystals}, {lo}, {hi})"],
+                   env=dict(os.environ, CFB200_SIDE_STREAM="0"), check=True, timeout=300)
+    wanted = [[x.cuda() for x in w] for w in torch.load(path)]
+    model, tb, sets = _model_and_two_batches(method, crystals, lo, hi)
+    for pos, want in zip(sets, wanted):
+        tb.pos.copy_(pos)
+        for x, y in zip(_seeded(lambda: _gradients(model, tb)), want):
+            assert torch.equal(x, y)
+    torch.cuda.synchronize()
     graph = torch.cuda.CUDAGraph()
     with torch.cuda.graph(graph):
-        got = predict()
-    for _ in range(3):
-        tb.pos.copy_(tb.pos.clone())
-        graph.replay()
-        torch.cuda.synchronize()
-        assert torch.equal(got, want)
+        got = _seeded(lambda: _gradients(model, tb))
+    _replays_follow(tb, sets, wanted, graph, got)
