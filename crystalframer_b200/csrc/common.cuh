@@ -70,10 +70,13 @@ __device__ __forceinline__ float ex2_approx(float x)
     return y;
 }
 
-// Launches ahead: a kernel may be brought to the SMs while the last blocks of the one before it in the stream still run, and
-// waits there until everything before it has finished and its writes can be seen.  Every such kernel begins with that wait,
-// in all its blocks, before anything else that touches global memory; so a kernel that has finished has all its predecessors
-// behind it, as in any stream.  What it saves is the gap between two kernels, 1.7 us in a step of some 120 launches:
+// Launches ahead: a kernel may be brought to the SMs before the one in front of it in the stream has been retired, and waits
+// there until everything before it has finished and its writes can be seen.  Every such kernel begins with that wait, in all
+// its blocks, before anything else that touches global memory; so a kernel that has finished has all its predecessors behind
+// it, as in any stream.  No kernel here says by itself when the next one may come (griddepcontrol.launch_dependents): that is
+// when all of its blocks have ended, so what overlaps is the end of a grid, its flush and the next one's launch, never blocks
+// of the two.  (A kernel that did say so would share the SMs with the next one's blocks, and those of tc_linear.cu allocate
+// tensor memory before they wait.)  What it saves is the gap between two kernels, 1.7 us in a step of some 120 launches:
 // training step of 256 crystals 3.70 -> 3.52 ms, of 128 with the lightweight recipe 2.39 -> 2.19, prediction of 256
 // 2.21 -> 2.09.  (The weight gradients' kernels, the first behind a side stream's fork, are launched as usual.)
 __device__ __forceinline__ void wait_for_predecessors() { asm volatile("griddepcontrol.wait;" ::: "memory"); }

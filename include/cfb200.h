@@ -511,8 +511,10 @@ int cfb200_batch_geometry_pairwise(const float* pos, const float* tvecs, const i
  * reference computes with torch.nn.functional.linear (models/indexed_lattice_multi_head_attention_cuda.py:869,
  * :987-988; models/indexed_latticeformer_encoder.py:888-890).  weight_is_kn = 0: W is (N,K) as torch stores a
  * Linear weight (y = x W^T); 1: W is (K,N) (y = x W, the data gradient of the same layer).  K and N must be
- * multiples of 4 and all pointers 16-byte aligned.  Runs on the tensor cores (tcgen05, three-product TF32
- * split with FP32 accumulation) when N is a multiple of 128 and K of 32, else on the FP32 pipe. */
+ * multiples of 4 and all pointers 16-byte aligned.  Runs on the tensor cores when
+ * M >= 512, N is a multiple of 64 and K of 32 (tcgen05: operands split into three bf16 parts, six products, FP32
+ * accumulation, contractions of more than 512 terms in runs that are added in FP32), else on the FP32 pipe: the
+ * rounding of a result, not its distance from the exact one, changes at 512 rows. */
 int cfb200_linear(const float* x, const float* weight, const float* bias, const float* residual, int64_t M,
                   int64_t N, int64_t K, int relu, int weight_is_kn, float* y, void* stream);
 

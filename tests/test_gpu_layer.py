@@ -370,8 +370,8 @@ def test_sharded_step_equals_whole_batch():
                                       (129, 512, 128, 1), (64, 96, 36, 0)])
 def test_dense_layer_kernels(M, N, K, kn):
     """cfb200_linear (the kernels behind the layer's dense parts) against float64 matmul: plain, with bias +
-    residual + ReLU, for torch-layout and transposed weights, at sizes with ragged last tiles.  The last case has a
-    shape the tensor-core kernel does not cover and runs on the FP32 pipe."""
+    residual + ReLU, for torch-layout and transposed weights, at sizes with ragged last tiles.  Those of 512
+    rows and more run on the tensor cores, the others on the FP32 pipe (the last one also for its shape)."""
     dev = cuda()
     from crystalframer_b200 import _lib, cuda_funcs as F
     F.compile_kernels(2, 8, 16, 64, 64, 16, True, 0, 1.0, 4.0, 1.0, 1.0, 0.0)
