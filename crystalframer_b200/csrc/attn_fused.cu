@@ -103,10 +103,11 @@ __host__ __device__ constexpr int fw_rows(int mode) { return mode == 1 ? 4 : (mo
 // 228 us, 12 x 2 242 us; mode 1: 10 x 2 335 us, 5 x 4 352 us, 12 x 2 (80 registers) 374 us; mode 0: within 2 %.
 __host__ __device__ constexpr int fw_warps(int mode) { return mode == 0 ? 16 : (mode == 1 ? 10 : 6); }
 __host__ __device__ constexpr int fw_blocks(int mode) { return mode == 2 ? 4 : 2; }
-__host__ __device__ constexpr size_t fw_smem_bytes(int AH, int mode)
+// EACH: mode 2 with lane sums formed pair by pair (see drain)
+__host__ __device__ constexpr size_t fw_smem_bytes(int AH, int mode, bool each)
 {
     return sizeof(float) * (kAtHd * fw_k(AH) + fw_warps(mode) * (32 * kFwRec + 5 * kFwStage + fw_rows(mode) * fw_k(AH) +
-                                                                      (mode == 2 && AH > 0 ? 2 * kFwWait * kFwWaitLd : 0)));
+                                                                      (mode == 2 && !each ? 2 * kFwWait * kFwWaitLd : 0)));
 }
 // translations whose weight is below exp(-24) = 4e-11 of the nearest one's do not enter the normaliser: the 125 of a
 // box together stay below a tenth of its last bit
@@ -308,7 +309,7 @@ __device__ __forceinline__ void fw_gaussians(const FwLane& L, const float4* R, c
     }
 }
 
-template <int AH, bool TASKS, int MODE>
+template <int AH, bool TASKS, int MODE, bool EACH>
 __global__ void __launch_bounds__(fw_warps(MODE) * 32, fw_blocks(MODE)) attn_tile_kernel(const AtArgs A, const Params P)
 {
     wait_for_predecessors();
@@ -452,10 +453,12 @@ __global__ void __launch_bounds__(fw_warps(MODE) * 32, fw_blocks(MODE)) attn_til
         if constexpr (MODE == 0) pooled([](const int, const float) { return 0.f; });
 
         // Backward: a pair's two sums over the lanes.  A butterfly per pair is seven dependent shuffles; eight pairs at once
-        // (lane = pair, quarter of the lanes) are 30 instructions, and the sums go to the lanes that hold the pairs.  Backward
-        // with the column pass, butterflies / eight at once: with frames 64 cells of 100-200 atoms 2.11 / 2.07 ms, 256
-        // log-normal crystals 0.51 / 0.51; but without frames 1.505 / 1.499, and in small cells, where nothing covers the wait
-        // for the other pairs, 256 crystals 0.262 / 0.300, 1 024 0.768 / 0.842: there each pair has its butterfly.
+        // (lane = pair, quarter of the lanes) are 30 instructions, and the sums go to the lanes that hold the pairs.  What either
+        // gives depends on the instance (EACH: butterflies), us per launch, butterflies / eight at once.  Frames, task table: 64
+        // cells of 100-200 atoms 1 992 / 1 936, 256 log-normal crystals 399 / 412; frames, no table, with the column pass: 2 103 /
+        // 2 071, 511 / 513.  Plain, task table: 1 377 / 1 308, 16 cells 333 / 321, cells of 20-100 atoms 322 / 323, of 50 249 /
+        // 244, but 256 log-normal crystals 220 / 238, 1 024 710 / 750, 256 of 4-16 atoms 209 / 225; plain, no table, with the
+        // column pass: 1 505 / 1 499, 262 / 300, 769 / 843.
         int waiting_pairs = 0, slot = -1;
         auto drain = [&]() {
             __syncwarp();
@@ -476,7 +479,7 @@ __global__ void __launch_bounds__(fw_warps(MODE) * 32, fw_blocks(MODE)) attn_til
         // the tile's pair j is complete: into the pooled sums, and into the row that waits for its projection
         auto flush = [&](const int j) {
             if constexpr (BACK) {
-                if constexpr (AH == 0) {
+                if constexpr (EACH) {
                     // both sums over the lanes at once: the lower half of the warp takes B, the upper A
                     const bool up = lane & 16;
                     float r = (up ? accA : accB) + __shfl_xor_sync(0xffffffffu, up ? accB : accA, 16);
@@ -1656,11 +1659,11 @@ int attn_plan(const int32_t* order, const int32_t* split, const float* a_ik, con
     return cudaGetLastError() == cudaSuccess ? CFB200_OK : CFB200_E_CUDA;
 }
 
-template <int AH, bool TASKS, int MODE>
+template <int AH, bool TASKS, int MODE, bool EACH = false>
 static int launch_tile(const AtArgs& A, const Params& P, cudaStream_t st)
 {
-    auto kern = attn_tile_kernel<AH, TASKS, MODE>;
-    constexpr size_t smem = fw_smem_bytes(AH, MODE);
+    auto kern = attn_tile_kernel<AH, TASKS, MODE, EACH>;
+    constexpr size_t smem = fw_smem_bytes(AH, MODE, EACH);
     static std::atomic<bool> attr_done[64];   // per instantiation and device
     int dev = 0;
     cudaGetDevice(&dev);
@@ -1721,7 +1724,11 @@ static int launch_tile(const AtArgs& A0, const Params& P, cudaStream_t st)
     A.vec_list = aligned(A.list);
     if (!A.counters_zeroed && cudaMemsetAsync(A.counters, 0, sizeof(int) * P.H, st) != cudaSuccess) return CFB200_E_CUDA;
     const bool tasks = A.tasks != nullptr;
-    if (A.W[1] == nullptr) return tasks ? launch_tile<0, true, MODE>(A, P, st) : launch_tile<0, false, MODE>(A, P, st);
+    if (A.W[1] == nullptr) {
+        // the plain backward: sums of eight pairs at once pay in big cells (more than 32 pairs per atom), with the task table
+        if (MODE == 2 && tasks && A.E <= 32 * A.N) return launch_tile<0, true, MODE, MODE == 2>(A, P, st);
+        return tasks ? launch_tile<0, true, MODE>(A, P, st) : launch_tile<0, false, MODE, MODE == 2>(A, P, st);
+    }
     if (P.angle_dim <= 32) return tasks ? launch_tile<1, true, MODE>(A, P, st) : launch_tile<1, false, MODE>(A, P, st);
     return tasks ? launch_tile<2, true, MODE>(A, P, st) : launch_tile<2, false, MODE>(A, P, st);
 }
