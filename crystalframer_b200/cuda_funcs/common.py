@@ -43,12 +43,20 @@ def f32c(t):
     return t.clone() if t.data_ptr() & 15 else t
 
 
-def stamp(*tensors):
-    """What a result that is kept for these tensors is compared by: where their memory is and how it is read, and the version
-    of its contents (none that could ever be equal for tensors that do not count theirs).  It holds as long as whoever keeps it
-    also keeps the tensors, or aliases of them: else another tensor could come to lie at the address."""
-    return tuple(None if t is None else (t.data_ptr(), object() if t.is_inference() else t._version, t.shape, t.stride(), t.dtype)
-                 for t in tensors)
+def kept(*tensors):
+    """What a result that is kept for these tensors holds to tell whether it still stands (unchanged): the tensors, or aliases of
+    them, so that no other tensor can take their place in memory, and where that is and the version of its contents (none for
+    tensors that do not count theirs: they are never found unchanged)."""
+    return tuple((t, t.data_ptr(), None if t.is_inference() else t._version) for t in tensors)
+
+
+def unchanged(entries, *tensors):
+    for (t, address, version), u in zip(entries, tensors):
+        if version is None or u.is_inference() or u.data_ptr() != address or u._version != version:
+            return False
+        if u is not t and (u.shape != t.shape or u.stride() != t.stride() or u.dtype != t.dtype):
+            return False
+    return True
 
 
 _pair_cache = {}
@@ -104,9 +112,8 @@ def pair_geometry(rpos_ij_e, tvecs_n, batch_i, edge_ij_e, cutoff):
     if rng <= 0:
         return None, None, 0
     key = id(rpos_ij_e)
-    sig = (rng, stamp(rpos_ij_e, tvecs_n, batch_i, edge_ij_e))
     hit = _pair_cache.get(key)
-    if hit is not None and hit[0]() is rpos_ij_e and hit[1] == sig:
+    if hit is not None and hit[0]() is rpos_ij_e and hit[1] == rng and unchanged(hit[4], rpos_ij_e, tvecs_n, batch_i, edge_ij_e):
         return hit[2], hit[3], rng
     _pair_cache.pop(key, None)
     dev = rpos_ij_e.device
@@ -121,5 +128,7 @@ def pair_geometry(rpos_ij_e, tvecs_n, batch_i, edge_ij_e, cutoff):
                 _lib.ptr(cache), _lib.ptr(plist))
     for k in [k for k, v in _pair_cache.items() if v[0]() is None]:      # lists are large: drop dead batches at once
         del _pair_cache[k]
-    _pair_cache[key] = (weakref.ref(rpos_ij_e), sig, cache, plist, tvecs_n.detach(), batch_i.detach(), edge_ij_e.detach())
+    # (aliases: the entry goes when the positions do, and a caller's pair list may hold on to those)
+    _pair_cache[key] = (weakref.ref(rpos_ij_e), rng, cache, plist,
+                        kept(*(t.detach() for t in (rpos_ij_e, tvecs_n, batch_i, edge_ij_e))))
     return cache, plist, rng

@@ -17,7 +17,7 @@ from . import _lib
 from . import fused_layer
 from .attention import CrystalformerMultiheadAttentionCUDA, gauss_scale_ready
 from .cuda_funcs import compile_kernels, register_csr
-from .cuda_funcs.common import stamp
+from .cuda_funcs.common import kept, unchanged
 from .cuda_funcs.kernel_manager import KernelManager
 from .latticeformer_params import LatticeformerParams
 
@@ -180,14 +180,13 @@ class CrystalformerEncoderLayerCUDA(Module):
         # the layers of a batch share its geometry, which hangs on the pair list; any other tensor may have been exchanged or
         # written to since
         cfg = KernelManager.config
-        sig = (meta["cutoff"], cfg and (cfg.lattice_range, cfg.minimum_range), stamp(pos_ij, trans, batch, edges, rvecs))
+        how = (meta["cutoff"], cfg and (cfg.lattice_range, cfg.minimum_range))
         geo = getattr(edges, "_cf_geometry", None)
-        if geo is None or geo.made_from != sig:
+        if geo is None or geo.made_how != how or not unchanged(geo.made_from, edges, pos_ij, trans, batch, rvecs):
             rvlen = torch.norm(rvecs, 2, dim=-1).contiguous() if meta["cutoff"] != 0.0 else None
             geo = fused_layer.LayerGeometry.from_tensors(pos_ij.contiguous(), trans.contiguous(), batch.contiguous(),
                                                          edges.contiguous(), rvlen, meta["cutoff"])
-            geo.made_from = sig
-            geo._keep += [t.detach() for t in (pos_ij, trans, batch, rvecs)]        # the stamp's addresses stay theirs
+            geo.made_how, geo.made_from = how, kept(edges.detach(), pos_ij, trans, batch, rvecs)
             edges._cf_geometry = geo
         return self.fused_apply(x, geo, meta)
 

@@ -73,7 +73,7 @@ class LayerGeometry:
         self.N = self.E = self.B = 0
         self.cache_range = 0
         self._keep = []
-        self.made_from = None      # what a caller that keeps this object compares it by
+        self.made_how = self.made_from = None      # what a caller that keeps this object compares it by
         self._ws = None
         self._plans = {}           # sizes of a layer's buffers on this batch, by what they depend on (see plan)
 
