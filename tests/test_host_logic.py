@@ -257,3 +257,19 @@ def test_free_memory_is_asked_for_rarely(monkeypatch):
     free[0] = 1 << 40
     monkeypatch.setattr(torch, "empty", full)
     assert common.allocate_pair_list(5, dev) is None and common._FREE_MEMORY == {}
+
+
+def test_what_is_kept_for_tensors_notices_writes_and_exchanges():
+    """kept / unchanged: the same tensors, and fresh views of them, are found unchanged; written to, exchanged, cut or transposed
+    ones, and tensors that do not count their versions, are not."""
+    from crystalframer_b200.cuda_funcs.common import kept, unchanged
+    a, b = torch.arange(12.0).view(3, 4), torch.arange(9.0).view(3, 3)
+    entries = kept(a, b.detach())
+    assert unchanged(entries, a, b) and unchanged(entries, a.view(3, 4), b[:])
+    assert not unchanged(entries, a.clone(), b) and not unchanged(entries, a, b[:2]) and not unchanged(entries, a, b.t())
+    assert not unchanged(entries, a, b.view(torch.int32))
+    b.view(-1)[0] = 5.0                                     # a write through a view counts
+    assert not unchanged(entries, a, b)
+    with torch.inference_mode():
+        c = torch.ones(3)
+        assert not unchanged(kept(c), c)
